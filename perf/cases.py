@@ -237,3 +237,56 @@ def tolerance(case):
     if kind == "all_reduce":
         return {"rel": 1.6e-2, "max": 0.1} if dt == "bf16" else {"rel": 2e-3, "max": 1e-2}    # 4.0e-3, 2.3e-2; 3.9e-4
     return {"rel": 7e-3, "max": 1.6e-2} if dt == "bf16" else {"rel": 9e-4, "max": 2e-3}       # 1.7e-3, 3.9e-3; 2.1e-4
+
+
+# ---- the same results in 64 bits ------------------------------------------------------------------------------------
+def exact(case, seed):
+    """What ``run`` returns for these inputs, from plain torch in float64 and the definitions of the operations."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kind = case["kind"]
+    if kind in ("all_scatter", "all_reduce", "gemm"):
+        a = _operand((case["m"], case["k"]), case["dtype"], gen)
+        bt = _operand((case["n"], case["k"]), case["dtype"], gen, 1.0 / math.sqrt(case["k"]))
+        c = a.double() @ bt.double().t()
+        if case["dtype"] == "int8":   # sums below 2^28, exact in float64; the low 8 bits of each
+            c = c.to(torch.int64).to(torch.int8)
+        return c
+    if kind == "attention":
+        t, w = case["batch"] * case["seq"], case["heads"] * HEAD
+        return _exact_attention(_operand((t, 3 * w), case["dtype"], gen).double(), case["batch"], case["seq"], case["heads"],
+                                case["causal"])
+    if kind == "decoder":
+        cfg = _config(case, seed)
+        return _exact_decoder(_operand((cfg.tokens, cfg.hidden), "bf16", gen).double(), cfg)
+    src = torch.randn(case["chunks"] * case["chunk_bytes"] // 4, generator=gen, device="cuda").double()
+    return src, 2 * src
+
+
+def _exact_attention(qkv, batch, seq, heads, causal):
+    q, k, v = qkv.view(batch, seq, 3, heads, HEAD).unbind(2)
+    out = torch.empty((batch, seq, heads, HEAD), dtype=torch.float64, device=qkv.device)
+    later = torch.ones((seq, seq), dtype=torch.bool, device=qkv.device).triu(1)   # keys after the query
+    for b in range(batch):
+        for h in range(heads):
+            s = q[b, :, h] @ k[b, :, h].t() / math.sqrt(HEAD)
+            if causal:
+                s.masked_fill_(later, -math.inf)
+            out[b, :, h] = torch.softmax(s, -1) @ v[b, :, h]
+    return out.view(batch * seq, heads * HEAD)
+
+
+def _exact_decoder(x, cfg):
+    h, i = cfg.hidden, cfg.intermediate
+
+    def norm(t):   # the norms' weights are ones
+        return t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + cfg.eps)
+    for layer in range(cfg.n_layers):
+        gen = torch.Generator(device="cuda").manual_seed(cfg.seed * 1000 + layer)
+        wq, wk, wv, wo, wg, wu, wd = [(torch.randn(s, generator=gen, device="cuda") * cfg.std).to(torch.bfloat16).double()
+                                      for s in ((h, h), (h, h), (h, h), (h, h), (i, h), (i, h), (h, i))]
+        n = norm(x)
+        a = _exact_attention(torch.cat([n @ wq.t(), n @ wk.t(), n @ wv.t()], 1), cfg.batch, cfg.seq, cfg.n_heads, True)
+        x = x + a @ wo.t()
+        n = norm(x)
+        x = x + (torch.nn.functional.silu(n @ wg.t()) * (n @ wu.t())) @ wd.t()
+    return x
