@@ -17,6 +17,7 @@ times; flags are cumulative counters, so nothing is reset between calls.
 from __future__ import annotations
 
 import ctypes
+import os
 from typing import List, Optional, Sequence, Union
 
 import torch
@@ -71,6 +72,16 @@ def _lib():
         lib.iris_gemm_plan_cta_group.argtypes = [ctypes.c_void_p]
         lib.iris_gemm_plan_launch.restype = ctypes.c_int
         lib.iris_gemm_plan_launch.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+        # one rank: csrc/kernels/gemm_local.cu
+        ptr, i32, i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
+        operands = [ptr, i64, ptr, i64, ptr, i64, i32, i32, i32, i32, i32, ptr, ctypes.c_uint64, i32, i32, i32, i32]
+        lib.iris_gemm_local_last_error.restype = ctypes.c_char_p
+        lib.iris_gemm_local_create.restype = ptr
+        lib.iris_gemm_local_create.argtypes = operands
+        lib.iris_gemm_local.argtypes = operands + [ptr]
+        lib.iris_gemm_local_launch.argtypes = [ptr, ptr]
+        lib.iris_gemm_local_destroy.argtypes = [ptr]
+        lib.iris_gemm_local_info.argtypes = [ptr, ctypes.POINTER(i32)]
         if lib.iris_gemm_desc_size() != ctypes.sizeof(_Desc):
             raise RuntimeError("IrisGemmDesc layout mismatch between Python and the native library")
         lib._gemm_typed = True
@@ -194,6 +205,12 @@ class FusedGemm:
         self.a, self.bt = a_use, bt
         dev = c0.device
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        # One rank: nothing to exchange, so the product goes straight into the output (csrc/kernels/gemm_local.cu), unless
+        # the caller asks for a schedule of the fused kernel or for its trace.
+        self.local = (self.world == 1 and not trace and not nvls and "IRIS_STREAM_K" not in os.environ and all(
+            x is None for x in (ctas_per_rank, group_m, cta_group, stream_k, push, ksplit, bn, tail_split, push_kind)))
+        if self.local:
+            stream_k = False
         # tile shape, persistent grid, schedule, flag count and buffer layout: a pure function of the problem
         pl = plan_gemm(self.M, self.N, self.K, self.world, self.num_local, mode, sms, ag=self.ag, cta_group=cta_group,
                        ctas_per_rank=ctas_per_rank, group_m=group_m, stream_k=stream_k, push=push, ksplit=ksplit,
@@ -320,6 +337,17 @@ class FusedGemm:
         if not self._plan:
             raise RuntimeError("fused GEMM plan: " + lib.iris_gemm_last_error().decode())
         self.ctas_per_rank = lib.iris_gemm_plan_ctas_per_rank(self._plan)  # what fits on the device
+        if self.local:   # the fused plan has vetted the arguments; what runs is the one-rank kernel
+            lib.iris_gemm_plan_destroy(self._plan)
+            a0, b0, o0 = a_use[0], bt[0], self.out[0]
+            self._plan = lib.iris_gemm_local_create(
+                a0.data_ptr(), a0.stride(0), b0.data_ptr(), b0.stride(0), o0.data_ptr(), o0.stride(0), self.M, self.N,
+                self.K, d.dtype, c0.gpu_id, c0.status.data_ptr(), d.timeout_ns, -1, 0, 0, 0)
+            if not self._plan:
+                raise RuntimeError("GEMM plan: " + lib.iris_gemm_local_last_error().decode())
+            info = (ctypes.c_int * 6)()
+            lib.iris_gemm_local_info(self._plan, info)
+            self.swap, self.cta_group, self.bn, self.ksplit, self.ctas_per_rank = list(info)[:5]
         self.calls = 0
         self.launches = 0
         # Construction is collective.  The flags were zeroed on this rank's stream just now; a peer that is already
@@ -331,6 +359,12 @@ class FusedGemm:
     def __call__(self, stream=None) -> List[torch.Tensor]:
         c0 = self.ctxs[0]
         st = torch.cuda.current_stream(c0.device).cuda_stream if stream is None else stream
+        if self.local:
+            self.calls += 1
+            if _lib().iris_gemm_local_launch(self._plan, ctypes.c_void_p(st)) != 0:
+                raise RuntimeError("GEMM launch: " + _lib().iris_gemm_local_last_error().decode())
+            self.launches += 1
+            return self.out
         if self.mode == "reduce" and not self._zero_in_kernel:
             for o in self.out[:self.num_local]:
                 o.zero_()  # partial sums are added into the output: it has to start at zero
@@ -379,8 +413,11 @@ class FusedGemm:
         ``examples/07_gemm_all_scatter/matmul_wrapper.py:152-155``).  Empty when the build record is missing."""
         from .. import _build
         pull = self.mode in ("one_shot", "two_shot")
-        want = (f"fused_gemm_kernel<{self.cta_group}, {'true' if pull else 'false'}, "
-                f"{DTYPES[_TORCH_DTYPES[self.dtype]]}>")
+        if self.local:
+            want = f"local_gemm_kernel<{DTYPES[_TORCH_DTYPES[self.dtype]]}, {self.cta_group}>"
+        else:
+            want = (f"fused_gemm_kernel<{self.cta_group}, {'true' if pull else 'false'}, "
+                    f"{DTYPES[_TORCH_DTYPES[self.dtype]]}>")
         for name, res in _build.kernel_resources().items():
             if want in name:
                 return dict(res, kernel=want)
@@ -394,7 +431,7 @@ class FusedGemm:
 
     def close(self) -> None:
         if getattr(self, "_plan", None):
-            _lib().iris_gemm_plan_destroy(self._plan)
+            (_lib().iris_gemm_local_destroy if self.local else _lib().iris_gemm_plan_destroy)(self._plan)
             self._plan = None
 
     def rebuild(self) -> "FusedGemm":
@@ -460,7 +497,8 @@ def gemm_all_reduce(ctxs, a, bt, variant: str = "one_shot", **kw) -> FusedGemm:
     to every rank; needs ``M`` to be a multiple of ``world x 128``)."""
     if variant == "auto":
         variant, auto_kw = auto_all_reduce_variant(a[0].shape[0], world_of(ctxs))
-        kw = dict(auto_kw, **kw)
+        # (one rank has nothing to reduce: the op picks its own schedule, see FusedGemm)
+        kw = dict(auto_kw, **kw) if world_of(ctxs) > 1 else kw
     if variant == "atomic":
         return FusedGemm(ctxs, a, bt, "reduce", store_all=True, **kw)
     if variant in ("one_shot", "two_shot"):
@@ -492,16 +530,34 @@ _private_ctx = {}
 def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
          cta_group: Optional[int] = None, bn: Optional[int] = None, tail_split: Optional[bool] = None) -> torch.Tensor:
     """Single-GPU ``a @ bt.T`` on the tcgen05 kernel (world of one, no communication): bf16, fp16, float32 (as tf32)
-    or int8 (the low 8 bits of the integer sums)."""
+    or int8 (the low 8 bits of the integer sums).  Runs in stream order on the current stream; with an explicit schedule
+    (``cta_group``, ``bn``, ``tail_split``) it builds and releases a :class:`FusedGemm` and waits for it."""
     dev = a.device
     ctx = _private_ctx.get(dev)
     if ctx is None:
         with torch.cuda.device(dev):
             ctx = Iris.local_world(1, heap_size=64 << 20, backend="cuda", device=dev.index)[0]
         _private_ctx[dev] = ctx
-    n = as_kmajor_bt(bt).shape[0]
+    bt = as_kmajor_bt(bt)
+    n = bt.shape[0]
     if out is None:
         out = torch.empty((a.shape[0], n), dtype=a.dtype, device=dev)
+    if cta_group is None and bn is None and tail_split is None and "IRIS_STREAM_K" not in os.environ:
+        _check_operand(bt, "B")
+        _check_operand(a, "A", bt.dtype)
+        if a.shape[1] != bt.shape[1]:
+            raise ValueError(f"K mismatch: A has {a.shape[1]}, B has {bt.shape[1]}")
+        _check_operand(out, "output", bt.dtype)
+        stream = torch.cuda.current_stream(dev)
+        lib = _lib()
+        rc = lib.iris_gemm_local(a.data_ptr(), a.stride(0), bt.data_ptr(), bt.stride(0), out.data_ptr(), out.stride(0),
+                                 a.shape[0], n, a.shape[1], DTYPES[_TORCH_DTYPES[bt.dtype]], dev.index or 0,
+                                 ctx.status.data_ptr(), 2000000000, -1, 0, 0, 0, stream.cuda_stream)
+        if rc != 0:
+            raise RuntimeError("GEMM: " + lib.iris_gemm_local_last_error().decode())
+        for t in (a, bt, out):   # the caller may let go of them, whatever stream they come from
+            t.record_stream(stream)
+        return out
     mark = ctx.mark()
     op = FusedGemm(ctx, [a], [bt], "store", out=[out], cta_group=cta_group, bn=bn, tail_split=tail_split)
     op()

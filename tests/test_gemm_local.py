@@ -1,0 +1,138 @@
+"""The one-rank GEMM kernel (``csrc/kernels/gemm_local.cu``): its choice of tile and split on the CPU, and on a GPU every
+form of it (operands swapped or not, single CTAs and pairs, tile widths, pieces of K) against a float64 product, at sizes
+with remainders in every dimension.
+
+Bounds: the operands are multiplied exactly and summed in fp32 (int8: in 32-bit integers), so a 16-bit result is off by
+its rounding, half a unit in the last of 8 (bf16) or 11 (fp16) bits, at most 2^-8 or 2^-11 of the value, plus the fp32 sums' K * 2^-24 of the sum of magnitudes; a tf32
+product rounds each operand to 11 bits, so every term is off by at most 2 * 2^-11 of its magnitude.  int8 is exact."""
+import ctypes
+import random
+
+import pytest
+import torch
+
+from iris_b200 import _native
+
+TYPES = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp32": torch.float32, "int8": torch.int8}
+CODE = {"bf16": 0, "fp16": 1, "fp32": 2, "int8": 3}
+SIZE = {"bf16": 2, "fp16": 2, "fp32": 4, "int8": 1}
+
+
+def _choice(m, n, k, dtype, sms=148):
+    lib = _native.kernels()
+    lib.iris_gemm_local_choice.restype = ctypes.c_double
+    v = [ctypes.c_int() for _ in range(4)]
+    t = lib.iris_gemm_local_choice(m, n, k, CODE[dtype], sms, *[ctypes.byref(x) for x in v])
+    return [x.value for x in v] + [t]
+
+
+@pytest.mark.skipif(not _native.kernels_available(), reason="native kernels not built")
+def test_choice_is_launchable_for_every_size():
+    rng = random.Random(3)
+    for _ in range(3000):
+        dtype = rng.choice(list(TYPES))
+        g = 16 // SIZE[dtype]
+        m = rng.choice([1, 2, 64, 128, 129, 256, 257, rng.randint(1, 40000)])
+        n, k = g * rng.randint(1, 4000 // g + 1), g * rng.choice([1, 2, 8, 9, rng.randint(1, 20000 // g + 1)])
+        swap, cg, tn, split, t = _choice(m, n, k, dtype, rng.choice([148, 132, 16, 1]))
+        kblocks = -(-k * SIZE[dtype] // 128)
+        assert swap in (0, 1) and cg in (1, 2) and t > 0
+        assert 16 <= tn <= 256 and tn % (32 if dtype == "int8" else 16) == 0
+        assert 1 <= split <= kblocks and split * cg <= 8
+        assert not (swap and m > 256)
+
+
+def _operand(shape, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    if dtype == "int8":
+        return torch.randint(-128, 128, shape, generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
+    return torch.randn(shape, generator=g, device="cuda").to(TYPES[dtype])
+
+
+def _check(got, a, bt):
+    exact = a.double() @ bt.double().t()
+    if got.dtype == torch.int8:
+        assert torch.equal(got, exact.to(torch.int64).to(torch.int8))
+        return
+    size = a.double().abs() @ bt.double().abs().t()
+    unit = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -24}[got.dtype]
+    bound = unit * exact.abs() + a.shape[1] * 2.0 ** -24 * size + 1e-30
+    if got.dtype == torch.float32:
+        bound = bound + 2.0 * 2.0 ** -11 * size
+    assert bool(((got.double() - exact).abs() <= 1.01 * bound).all())
+
+
+def _run(a, bt, out, swap=-1, cg=0, tn=0, split=0, stream=None):
+    from iris_b200.ops import gemm as G
+    lib = G._lib()
+    status = torch.zeros(16, dtype=torch.int32, device="cuda")
+    name = [t for t, d in TYPES.items() if d == a.dtype][0]
+    rc = lib.iris_gemm_local(a.data_ptr(), a.stride(0), bt.data_ptr(), bt.stride(0), out.data_ptr(), out.stride(0),
+                             a.shape[0], bt.shape[0], a.shape[1], CODE[name], 0, status.data_ptr(), 2000000000, swap, cg,
+                             tn, split, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, lib.iris_gemm_local_last_error().decode()
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", list(TYPES))
+@pytest.mark.parametrize("cg,split", [(1, 1), (2, 1), (1, 2), (1, 3), (1, 8), (2, 2), (2, 3), (2, 4)])
+@pytest.mark.parametrize("swap", [0, 1])
+def test_every_form_against_float64(dtype, cg, split, swap):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    g = 16 // SIZE[dtype]
+    for i, (m, n, k) in enumerate([(1, g, 64 * g), (17, 40 * g, 81 * g), (130, 31 * g, 64 * g), (300, 65 * g, 145 * g)]):
+        for tn in (32, 96, 256) if dtype == "int8" else (16, 48, 112, 256):
+            a, bt = _operand((m, k + g), dtype, i)[:, :k], _operand((n, k), dtype, i + 9)   # a: rows at a pitch of k + g
+            frame = torch.full((m + 2, n + 4 * g), 3, dtype=TYPES[dtype], device="cuda")
+            out = frame[1:m + 1, g:g + n]
+            _run(a, bt, out, swap, cg, tn, split)
+            _check(out, a, bt)
+            frame[1:m + 1, g:g + n] = 3
+            assert bool((frame == 3).all()), "wrote outside the output"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(1, 2048, 4096), (64, 1456, 1448), (129, 2504, 1736), (2500, 2048, 512)])
+@pytest.mark.parametrize("dtype", ["bf16", "int8"])
+def test_choice_matches_and_repeats(m, n, k, dtype):
+    """What the rule picks is right, gives the same bits each time, and the same through ``gemm`` and a prepared op of any
+    collective form (one rank: all of them are the product)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import iris_b200 as iris
+    from iris_b200.ops import gemm as G
+    n, k = n // 16 * 16, k // 16 * 16
+    a, bt = _operand((m, k), dtype, 1), _operand((n, k), dtype, 2)
+    outs = [torch.empty((m, n), dtype=TYPES[dtype], device="cuda") for _ in range(2)]
+    for o in outs:
+        _run(a, bt, o)
+    _check(outs[0], a, bt)
+    assert torch.equal(outs[0], outs[1])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        c = G.gemm(a, bt)
+    side.synchronize()
+    assert torch.equal(c, outs[0])
+    ctx = iris.iris(256 << 20)
+    ops = [G.gemm_all_scatter(ctx, [a], [bt])]
+    if dtype == "bf16":
+        ops += [G.gemm_all_reduce(ctx, [a], [bt], variant=v) for v in ("auto", "atomic", "one_shot", "two_shot")]
+    for op in ops:
+        assert op.local
+        graph = torch.cuda.CUDAGraph()
+        op()
+        op.check()
+        assert torch.equal(op.out[0], outs[0])
+        op.out[0].zero_()
+        with torch.cuda.graph(graph):
+            op()
+        graph.replay()
+        op.check()
+        assert torch.equal(op.out[0], outs[0])
+        graph.reset()
+        op.close()
+    ctx.close()
