@@ -7,16 +7,24 @@
 // fp32 accumulation and softmax.  No counterpart in the reference (it has no model code); it replaces the library
 // attention call inside iris_b200/models/tp_block.py.
 //
-// One CTA per (batch, head, tile of 128 queries); it walks over the key tiles of 128 (causal: up to its own):
-//   warp 0      TMA producer: Q once, then K_j / V_j into a two-stage ring (cp.async.bulk.tensor, no multicast)
-//   warp 1      one thread issues tcgen05.mma:  S_j = Q K_j^T (128 x 128 x 128, both operands K-major) into one of
-//               two S accumulators in tensor memory, and O_j = P_j V_j (P from shared memory, V as an MN-major
-//               operand: V[key][d] is read as stored) into one of two O accumulators
-//   warps 2-9   softmax, two threads per query row (64 keys / 64 output columns each): tcgen05.ld of S_j, running
-//               maximum (over the whole row, read by both), exp2, row sum, P_j as 16-bit values into shared
-//               memory in the swizzled layout the MMA expects; then O_{j-1} is read from tensor memory and folded
-//               into the fp32 output row kept in registers (rescaled by exp2(m_old - m_new)).
-// While the softmax warps work on S_j the tensor cores already compute S_{j+1}.
+// A CTA works on two 128-row sides, A and B, at once, so that the tensor cores compute the scores of one side while the
+// other side is in its exponentials (the two take about the same time: 1024 cycles of MMAs and 1024 of ex2 per tile of
+// 128 x 128).  Two ways to fill the sides:
+//   pair    A and B are neighbouring tiles of 128 queries of one head and share every K / V tile: half the loads
+//   split   A and B are the same queries, A takes the even key tiles and B the odd ones, and the two partial outputs are
+//           merged at the end: half the serial chain, for problems whose query tiles do not fill the GPU
+// Persistent: a CTA takes its items from a fixed list, longest first and dealt out back and forth so that the sums come
+// out even, heads in groups whose K and V stay in L2.  Roles (320 threads):
+//   warps 0-3, 4-7  softmax of side A, B, one thread per query row: tcgen05.ld of the row of scores, maximum, exp2, row
+//                   sum, and P as 16-bit values back into tensor memory over the scores, where the MMA reads it as its A
+//                   operand.  O stays in tensor memory for all key tiles.  It is rescaled only when the running maximum
+//                   has grown by more than 2^8 since the scale in use was taken (rare after the first tiles; P is then at
+//                   most 256, which changes neither its relative rounding nor that of the fp32 sums).
+//   warp 8          TMA producer: Q tiles, and K / V tiles through a ring of five slots (no multicast)
+//   warp 9          one elected thread issues tcgen05.mma:  S = Q K^T, then O += P V (P from tensor memory, V as an
+//                   MN-major operand: V[key][d] is read as stored), alternating between the sides
+// Before: one 128-row tile per CTA, two threads per row reading the scores twice, P through shared memory, O folded
+// through registers after every tile.  8 x 2048 tokens x 32 heads, causal, bf16: 668 -> 333 us back to back (power-limited), 649 -> 280 us from a rest.
 //
 // Every wait is bounded by timeout_ns: on expiry the CTA records a status, every role leaves its loop, tensor memory
 // is released and the kernel returns.
@@ -40,15 +48,20 @@ namespace attn {
 using namespace iris::ptx;
 
 constexpr int D = 128;            // head dimension
-constexpr int BQ = 128;           // queries per CTA
+constexpr int BQ = 128;           // queries per side
 constexpr int BKV = 128;          // keys per tile
 constexpr int kTileBytes = 128 * 128 * 2;   // one 128 x 128 tile of 16-bit elements (two 64-column swizzle blocks)
 constexpr int kHalfBytes = kTileBytes / 2;  // one 64-column block: 128 rows x 128 bytes
-constexpr int kThreads = 320;          // TMA warp, MMA warp, eight softmax warps
-// shared memory: Q | K[2] | V[2] | P, then barriers
-constexpr int kSmemTiles = 6 * kTileBytes;
-constexpr int kXchgBytes = 256 * 4;         // row sums exchanged between the two halves at the end
-constexpr int kSmemBytes = kSmemTiles + 256 + kXchgBytes + 1024;
+constexpr int kThreads = 320;
+constexpr int kSlots = 5;              // K / V ring
+constexpr int kBarBytes = 1024;        // barriers and small shared words
+// shared memory: barriers | Q of side A | Q of side B (split: row maxima and sums) | ring
+constexpr int kSmemBytes = 1024 + kBarBytes + (2 + kSlots) * kTileBytes;
+static_assert(kSmemBytes <= 227 * 1024, "shared-memory budget");
+
+// A row's scale is renewed when its maximum has grown by more than this (log2): P is at most 2^8, far from the fp16
+// limit of 65504.
+constexpr float kRescaleStep = 8.f;
 
 enum Site : uint32_t { kSiteLoad = 90, kSiteMma = 91, kSiteSoftmax = 92 };
 
@@ -57,6 +70,40 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// Two fp32 operations in one instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+template <bool F16>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  if (F16) {
+    __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
+  __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&b);
+}
+
+// Scores of the keys after `row` become minus infinity.
+template <int N>
+__device__ __forceinline__ void mask_after(uint32_t* v, int row) {
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i > row) v[i] = 0xff800000u;
 }
 
 struct Params {
@@ -67,272 +114,479 @@ struct Params {
   uint64_t timeout_ns;
   int batch, seq, heads;
   int causal;
+  int blocks;            // items per head: query tiles (split) or pairs of them
+  int group;             // heads whose items are dealt out together
+  int items;
   float scale_log2;      // log2(e) / sqrt(128)
 };
 
-template <bool F16>
+// One item of the list: head `bh`, query tiles qa and qa + 1 (pair) or qa (split), n key tiles loaded, of which side A
+// uses na and side B nb (0: side B has nothing to do).
+struct Item {
+  int bh, qa, n, na, nb;
+};
+
+// Item of round r of CTA c, false past the end of the list.
+template <bool SPLIT>
+__device__ __forceinline__ bool item_of(const Params& p, int r, Item& it) {
+  const int g = gridDim.x;
+  const int idx = r * g + ((r & 1) ? g - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  if (idx >= p.items) return false;
+  const int per = p.group * p.blocks;
+  const int first = idx / per * p.group;
+  const int left = p.batch * p.heads - first;
+  const int hc = left < p.group ? left : p.group;
+  const int rank = idx % per;
+  it.bh = first + rank % hc;
+  const int q = p.blocks - 1 - rank / hc;      // longest rows of work first
+  const int nq = p.seq / BQ;
+  if (SPLIT) {
+    it.qa = q;
+    it.n = p.causal ? q + 1 : nq;
+    it.na = (it.n + 1) / 2;
+    it.nb = it.n / 2;
+  } else {
+    it.qa = 2 * q;
+    const bool b = it.qa + 1 < nq;
+    it.na = p.causal ? it.qa + 1 : nq;
+    it.nb = !b ? 0 : p.causal ? it.qa + 2 : nq;
+    it.n = it.nb > it.na ? it.nb : it.na;
+  }
+  return true;
+}
+
+template <bool F16, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid_constant__ Params p) {
-  constexpr int kFirstSoftmaxWarp = 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t q_s = smem_u32(smem);
-  const uint32_t k_s = q_s + kTileBytes;          // 2 stages
-  const uint32_t v_s = k_s + 2 * kTileBytes;      // 2 stages
-  const uint32_t p_s = v_s + 2 * kTileBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kSmemTiles);
-  const uint32_t bar0 = smem_u32(bars);
-  // 0 q_full | 1,2 k_full | 3,4 v_full | 5,6 kv_empty | 7,8 s_full | 9,10 s_free | 11 p_ready | 12,13 o_full | 14,15 o_free
-  auto bar = [&](int i) { return bar0 + 8u * i; };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 16);
-  volatile uint32_t* abort_flag = tmem_slot + 1;
-  volatile float* xchg = reinterpret_cast<volatile float*>(smem + kSmemTiles + 256);
+  const uint32_t bar0 = smem_u32(smem);
+  const uint32_t q_s = bar0 + kBarBytes;           // side A, side B
+  const uint32_t ring = q_s + 2 * kTileBytes;
+  // barriers; [x] = side
+  auto q_full = [&](int x) { return bar0 + 8u * (0 + x); };
+  auto q_empty = [&](int x) { return bar0 + 8u * (2 + x); };
+  auto s_full = [&](int x) { return bar0 + 8u * (4 + x); };    // scores complete (and everything issued before them)
+  auto p_ready = [&](int x) { return bar0 + 8u * (6 + x); };   // P in tensor memory, scores read, O rescaled
+  auto o_full = [&](int x) { return bar0 + 8u * (8 + x); };    // last product of the item complete
+  auto o_free = [&](int x) { return bar0 + 8u * (10 + x); };   // O has been read
+  const uint32_t merge_bar = bar0 + 8u * 12;                   // split: both sides' maxima and sums are in shared memory
+  const uint32_t drain_bar = bar0 + 8u * 13;
+  auto kv_full = [&](int s) { return bar0 + 8u * (16 + s); };
+  auto kv_empty = [&](int s) { return bar0 + 8u * (16 + kSlots + s); };
+  volatile uint32_t* words = reinterpret_cast<volatile uint32_t*>(smem + 8 * (16 + 2 * kSlots));
+  volatile uint32_t* tmem_slot = words;
+  volatile uint32_t* abort_flag = words + 1;
+  volatile uint32_t* never = words + 2;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = p.seq / BQ;
-  const int bh = blockIdx.x % (p.batch * p.heads);
-  const int qt = nq - 1 - blockIdx.x / (p.batch * p.heads);   // longest rows of work first
-  const int b = bh / p.heads, h = bh - b * p.heads;
-  const int nkv = p.causal ? qt + 1 : p.seq / BKV;
-  const int row0 = b * p.seq + qt * BQ;           // first query row in the [T, ...] matrices
-  const int xq = h * D, xk = (p.heads + h) * D, xv = (2 * p.heads + h) * D;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < 16; ++i) {
-      const bool by_warps = (i == 9 || i == 10 || i == 11 || i == 14 || i == 15);  // one arrival per softmax warp
-      mbar_init(bar(i), by_warps ? 8 : 1);
+  if (warp == 8 && elect_one()) {
+    prefetch_tensormap(&p.tm);
+    for (int x = 0; x < 2; ++x) {
+      mbar_init(q_full(x), 1);
+      mbar_init(q_empty(x), 1);
+      mbar_init(s_full(x), 1);
+      mbar_init(p_ready(x), 4);                  // one arrival per softmax warp of the side
+      mbar_init(o_full(x), 1);
+      mbar_init(o_free(x), SPLIT ? 8 : 4);     // split: both sides read both outputs
+    }
+    mbar_init(merge_bar, 8);
+    mbar_init(drain_bar, 1);
+    for (int s = 0; s < kSlots; ++s) {
+      mbar_init(kv_full(s), 1);
+      mbar_init(kv_empty(s), 1);
     }
     *abort_flag = 0;
+    *never = 0;
     mbar_fence_init();
-    prefetch_tensormap(&p.tm);
   }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);   // S[2] and O[2], 128 columns each
+  if (warp == 9) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);   // S (and P) of A and B, O of A and B: 128 columns each
     tmem_relinquish();
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_dependency_wait();
+  grid_dependency_launch();
 
-  if (warp == 0) {
-    if (lane == 0) {
-      mbar_expect_tx(bar(0), kTileBytes);
-      tma_load_2d(q_s, &p.tm, xq, row0, bar(0));
-      tma_load_2d(q_s + kHalfBytes, &p.tm, xq + 64, row0, bar(0));
-      for (int j = 0; j < nkv; ++j) {
-        const int st = j & 1;
-        if (j >= 2 && !mbar_wait(bar(5 + st), ((j >> 1) - 1) & 1, p.timeout_ns, abort_flag)) {
-          record_status(p.status, kTimeout, kSiteLoad, blockIdx.x, j, 0);
-          *abort_flag = 1;
-          break;
-        }
-        const int krow = b * p.seq + j * BKV;
-        mbar_expect_tx(bar(1 + st), kTileBytes);
-        tma_load_2d(k_s + st * kTileBytes, &p.tm, xk, krow, bar(1 + st));
-        tma_load_2d(k_s + st * kTileBytes + kHalfBytes, &p.tm, xk + 64, krow, bar(1 + st));
-        mbar_expect_tx(bar(3 + st), kTileBytes);
-        tma_load_2d(v_s + st * kTileBytes, &p.tm, xv, krow, bar(3 + st));
-        tma_load_2d(v_s + st * kTileBytes + kHalfBytes, &p.tm, xv + 64, krow, bar(3 + st));
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_idesc_f16_major(BQ, BKV, !F16, false, false);
-      constexpr uint32_t idesc_pv = umma_idesc_f16_major(BQ, D, !F16, false, true);   // V is MN-major
+  // Ring order of an item's tiles: K_0 .. K_{lead-1}, then V_i, K_{i+lead}, V_{i+1}, ...: the order in which the MMA
+  // thread needs them (pair: lead 1; split: lead 2, because each side starts with a key tile of its own).
+  const int lead = SPLIT ? 2 : 1;
+
+  if (warp == 8) {
+    if (elect_one()) {
       bool ok = true;
-      auto fail = [&](int j, int what) {
-        record_status(p.status, kTimeout, kSiteMma, blockIdx.x, j, what);
+      uint32_t pos = 0;                 // ring position
+      uint32_t qn[2] = {0, 0};          // Q tiles loaded per side
+      auto stop = [&](int what) {
+        record_status(p.status, kTimeout, kSiteLoad, blockIdx.x, pos, what);
         *abort_flag = 1;
         ok = false;
       };
-      // S_j = Q K_j^T into S accumulator j & 1
-      auto issue_qk = [&](int j) {
-        const int st = j & 1;
-        if (!mbar_wait(bar(1 + st), (j >> 1) & 1, p.timeout_ns, abort_flag)) return fail(j, 1);
-        if (j >= 2 && !mbar_wait(bar(9 + st), ((j >> 1) - 1) & 1, p.timeout_ns, abort_flag)) return fail(j, 2);
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kHalfBytes + (kk & 3) * 32;
-          umma_f16_ss(tmem + st * 128, umma_desc_k_sw128(q_s + off), umma_desc_k_sw128(k_s + st * kTileBytes + off),
-                      idesc_qk, kk ? 1u : 0u);
-        }
-        umma_commit(bar(7 + st));
+      auto load_tile = [&](uint32_t dst, int x, int y, uint32_t bar) {
+        mbar_expect_tx(bar, kTileBytes);
+        tma_load_2d(dst, &p.tm, x, y, bar);
+        tma_load_2d(dst + kHalfBytes, &p.tm, x + 64, y, bar);
       };
-      if (!mbar_wait(bar(0), 0, p.timeout_ns, abort_flag)) fail(0, 0);
-      if (ok) issue_qk(0);
-      for (int j = 0; j < nkv && ok; ++j) {
-        const int st = j & 1;
-        if (j + 1 < nkv) issue_qk(j + 1);
-        if (!ok) break;
-        if (!mbar_wait(bar(11), j & 1, p.timeout_ns, abort_flag)) { fail(j, 3); break; }          // P_j in shared memory
-        if (!mbar_wait(bar(3 + st), (j >> 1) & 1, p.timeout_ns, abort_flag)) { fail(j, 4); break; }  // V_j loaded
-        if (j >= 2 && !mbar_wait(bar(14 + st), ((j >> 1) - 1) & 1, p.timeout_ns, abort_flag)) { fail(j, 5); break; }
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t a_desc = umma_desc_k_sw128(p_s + (kk >> 2) * kHalfBytes + (kk & 3) * 32);
-          // 16 keys = two groups of 8 rows (1024 bytes apart); the second 64 columns of d are one half tile further on
-          const uint64_t b_desc = umma_desc_mn_sw128(v_s + st * kTileBytes + kk * 16 * 128, kHalfBytes, 1024);
-          umma_f16_ss(tmem + 256 + st * 128, a_desc, b_desc, idesc_pv, kk ? 1u : 0u);
+      auto load_kv = [&](int x, int y) {
+        if (!ok) return;
+        const int s = pos % kSlots;
+        const uint32_t use = pos / kSlots;
+        if (use > 0 && !mbar_wait(kv_empty(s), (use - 1) & 1, p.timeout_ns, abort_flag)) return stop(0);
+        load_tile(ring + s * kTileBytes, x, y, kv_full(s));
+        ++pos;
+      };
+      auto load_q = [&](int side, int x, int y) {
+        if (!ok) return;
+        const uint32_t use = qn[side]++;
+        if (use > 0 && !mbar_wait(q_empty(side), (use - 1) & 1, p.timeout_ns, abort_flag)) {
+          qn[side]--;
+          return stop(1);
         }
-        umma_commit(bar(12 + st));   // O_j complete (and P free again)
-        umma_commit(bar(5 + st));    // K_j / V_j stage free
+        load_tile(q_s + side * kTileBytes, x, y, q_full(side));
+      };
+      Item it;
+      for (int r = 0; r * (int)gridDim.x < p.items && ok; ++r) {
+        if (!item_of<SPLIT>(p, r, it)) continue;
+        const int b = it.bh / p.heads, h = it.bh - b * p.heads;
+        const int y0 = b * p.seq, xq = h * D, xk = (p.heads + h) * D, xv = (2 * p.heads + h) * D;
+        load_q(0, xq, y0 + it.qa * BQ);
+        load_kv(xk, y0);
+        if (!SPLIT && it.nb > 0) load_q(1, xq, y0 + (it.qa + 1) * BQ);
+        if (lead == 2 && it.n > 1) load_kv(xk, y0 + BKV);
+        for (int i = 0; i < it.n && ok; ++i) {
+          load_kv(xv, y0 + i * BKV);
+          if (i + lead < it.n) load_kv(xk, y0 + (i + lead) * BKV);
+        }
+      }
+      if (*abort_flag) {   // loads in flight still write into shared memory: wait for each, bounded
+        for (int s = 0; s < kSlots; ++s) {
+          const uint32_t n = (pos + kSlots - 1 - s) / kSlots;
+          if (n > 0) mbar_wait(kv_full(s), (n - 1) & 1, 200000, never);
+        }
+        for (int x = 0; x < 2; ++x)
+          if (qn[x] > 0) mbar_wait(q_full(x), (qn[x] - 1) & 1, 200000, never);
       }
     }
-  } else if (warp >= kFirstSoftmaxWarp) {
-    // ---- softmax + output: two threads per query row, one for keys / output columns 0..63, one for 64..127 ----
-    // (a warp may only read the 32 tensor-memory lanes of its quadrant, warp id % 4; warps 2-5 take the first half of
-    // the columns, warps 6-9 the second, so that every scheduler of the SM has two softmax warps to switch between)
-    const int quad = warp & 3;
-    const int half = (warp - kFirstSoftmaxWarp) >> 2;
-    const int row = quad * 32 + lane;
-    const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    float acc[64];
+  } else if (warp == 9) {
+    if (elect_one()) {   // elect.sync, not a lane number: see the same place in gemm_local.cu
+      constexpr uint32_t idesc_qk = umma_idesc_f16_major(BQ, BKV, !F16, false, false);
+      constexpr uint32_t idesc_pv = umma_idesc_f16_major(BQ, D, !F16, false, true);   // V is MN-major
+      bool ok = true;
+      uint32_t base = 0;                      // ring position of the current item's first tile
+      uint32_t sn[2] = {0, 0};                // tiles whose P has been waited for, per side
+      uint32_t qn[2] = {0, 0};                // Q tiles taken into use, per buffer
+      uint32_t on[2] = {0, 0};                // items begun, per side
+      bool ahead[2] = {false, false};         // the item's first scores are already under way
+      auto stop = [&](int what) {
+        record_status(p.status, kTimeout, kSiteMma, blockIdx.x, base, what);
+        *abort_flag = 1;
+        ok = false;
+      };
+      auto pos_k = [&](int i) { return (uint32_t)(i + (i >= lead ? i - lead + 1 : 0)); };
+      auto pos_v = [&](const Item& it, int i) { return (uint32_t)(i + (i + lead < it.n ? i + lead : it.n)); };
+      auto key_tile = [&](int x, int j) { return SPLIT ? 2 * j + x : j; };
+      // a tile's slot is free after its last use: side B's where both sides use it
+      auto last_use = [&](const Item& it, int x, int j) { return SPLIT || x == 1 || j >= it.nb; };
+      // S = Q K_j^T of side x; `first` = ring position of the item's first tile
+      auto scores = [&](const Item& it, uint32_t first, int x, int j) {
+        const int kt = key_tile(x, j);
+        const uint32_t pos = first + pos_k(kt);
+        const int s = pos % kSlots;
+        if (!mbar_wait(kv_full(s), (pos / kSlots) & 1, p.timeout_ns, abort_flag)) return stop(1);
+        tc_fence_after();
+        const uint64_t qd = umma_desc_k_sw128(q_s + (SPLIT ? 0 : x) * kTileBytes);
+        const uint64_t kd = umma_desc_k_sw128(ring + s * kTileBytes);
 #pragma unroll
-    for (int i = 0; i < 64; ++i) acc[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f, alpha_prev = 0.f;   // l_run: this half's part of the row sum
+        for (int kk = 0; kk < D / 16; ++kk) {
+          const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
+          umma_f16_ss(tmem + x * 128, qd + off, kd + off, idesc_qk, kk ? 1u : 0u);
+        }
+        umma_commit(s_full(x));
+        if (last_use(it, x, j)) umma_commit(kv_empty(s));
+        // the queries have been read for the last time by the item's last scores (of both sides, when they share them)
+        if (SPLIT ? kt == it.n - 1 : j == (x ? it.nb : it.na) - 1) umma_commit(q_empty(SPLIT ? 0 : x));
+      };
+      // waits for the item's queries on their first use
+      auto begin = [&](const Item& it, uint32_t first, int x) {
+        if (x == 0 || !SPLIT) {
+          if (!mbar_wait(q_full(x), qn[x] & 1, p.timeout_ns, abort_flag)) return stop(0);
+          ++qn[x];
+        }
+        scores(it, first, x, 0);
+      };
+      Item it, nx;
+      int r = 0;
+      auto fetch = [&](Item& to) {
+        for (; r * (int)gridDim.x < p.items; ++r)
+          if (item_of<SPLIT>(p, r, to)) {
+            ++r;
+            return true;
+          }
+        return false;
+      };
+      bool have = fetch(it);
+      while (have && ok) {
+        const bool more = fetch(nx);
+        const uint32_t next = base + 2 * it.n;
+        if (!ahead[0]) begin(it, base, 0);
+        if (ok && it.nb > 0 && !ahead[1]) begin(it, base, 1);
+        ahead[0] = ahead[1] = false;
+        const int steps = it.na > it.nb ? it.na : it.nb;
+        for (int j = 0; j < steps && ok; ++j) {
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const int n = x ? it.nb : it.na;
+            if (j >= n || !ok) continue;
+            if (j == 0) {
+              if (on[x] > 0 && !mbar_wait(o_free(x), (on[x] - 1) & 1, p.timeout_ns, abort_flag)) {
+                stop(2);
+                break;
+              }
+              ++on[x];
+            }
+            const uint32_t pos = base + pos_v(it, key_tile(x, j));
+            const int s = pos % kSlots;
+            if (!mbar_wait(kv_full(s), (pos / kSlots) & 1, p.timeout_ns, abort_flag) ||
+                !mbar_wait(p_ready(x), sn[x] & 1, p.timeout_ns, abort_flag)) {
+              stop(3);
+              break;
+            }
+            ++sn[x];
+            tc_fence_after();
+            // 16 keys = two groups of 8 rows (1024 bytes apart); the second 64 columns of d are one half tile further on
+            const uint64_t vd = umma_desc_mn_sw128(ring + s * kTileBytes, kHalfBytes, 1024);
+#pragma unroll
+            for (int kk = 0; kk < BKV / 16; ++kk)
+              umma_f16_ts(tmem + 256 + x * 128, tmem + x * 128 + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv,
+                          (j > 0 || kk > 0) ? 1u : 0u);
+            if (last_use(it, x, j)) umma_commit(kv_empty(s));
+            if (j + 1 < n) {
+              scores(it, base, x, j + 1);
+            } else {
+              umma_commit(o_full(x));
+              // go on with the next item on this side if its operands are there already
+              if (more && (x == 0 || (nx.nb > 0 && ahead[0]))) {   // (B never before A: see last_use)
+                const uint32_t np = next + pos_k(key_tile(x, 0));
+                const bool q_here = (x == 1 && SPLIT) || mbar_test(q_full(x), qn[x] & 1);
+                if (q_here && mbar_test(kv_full(np % kSlots), (np / kSlots) & 1)) {
+                  begin(nx, next, x);
+                  ahead[x] = true;
+                }
+              }
+            }
+          }
+        }
+        base = next;
+        it = nx;
+        have = more;
+      }
+      if (*abort_flag) {   // MMAs in flight still use shared and tensor memory
+        umma_commit(drain_bar);
+        mbar_wait(drain_bar, 0, 200000, never);
+      }
+    }
+  } else {
+    // ---- softmax: one thread per query row ----
+    const int x = warp >> 2;                       // side
+    const int row = (warp & 3) * 32 + lane;        // a warp reads the 32 tensor-memory lanes of its quadrant
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t s_t = tmem + lanes + x * 128, o_t = tmem + lanes + 256;
+    volatile float* merge = reinterpret_cast<volatile float*>(smem + kBarBytes + kTileBytes);   // split: Q of B is unused
     bool ok = true;
-    auto fail = [&](int j, int what) {
+    uint32_t sn = 0, dn = 0, bn = 0;               // score tiles, items (pair: of this side), items with a side B
+    auto stop = [&](int j, int what) {
       if (lane == 0) record_status(p.status, kTimeout, kSiteSoftmax, blockIdx.x, j, what);
       *abort_flag = 1;
       ok = false;
     };
-    // fold this thread's 64 columns of O_j (accumulator j & 1) into its output row: acc = acc * alpha + O_j
-    auto fold_o = [&](int j, float alpha) {
-      const int st = j & 1;
-      if (!mbar_wait(bar(12 + st), (j >> 1) & 1, p.timeout_ns, abort_flag)) return fail(j, 2);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {   // 32 columns at a time: the row of S or O is never whole in registers
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem + lane_addr + 256 + st * 128 + half * 64 + c * 32, v);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[c * 32 + i] = acc[c * 32 + i] * alpha + __uint_as_float(v[i]);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(14 + st));
-    };
-    for (int j = 0; j < nkv; ++j) {
-      const int st = j & 1;
-      if (!mbar_wait(bar(7 + st), (j >> 1) & 1, p.timeout_ns, abort_flag)) fail(j, 1);
-      const bool diag = p.causal && j == qt;
-      if (!ok) break;
-      // pass 1: maximum of the WHOLE row of scores (both halves: two more tensor-memory loads are cheaper than an
-      // exchange through shared memory and a barrier of all softmax warps in every tile)
-      float mx = -INFINITY;
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem + lane_addr + st * 128 + c * 32, v);
-        tmem_wait_ld();
-        if (diag) {   // keys after the query: minus infinity (ignored by the maximum, 0 after the exponential)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c * 32 + i > row) v[i] = 0xff800000u;
+    const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+    Item it;
+    for (int r = 0; r * (int)gridDim.x < p.items && ok; ++r) {
+      if (!item_of<SPLIT>(p, r, it)) continue;
+      const int n = x ? it.nb : it.na;
+      if (n == 0 && !SPLIT) continue;
+      const int qt = SPLIT ? it.qa : it.qa + x;
+      float m_run = -INFINITY, l_run = 0.f;
+#pragma unroll 1
+      for (int j = 0; j < n; ++j) {
+        if (!mbar_wait(s_full(x), sn & 1, p.timeout_ns, abort_flag)) {
+          stop(j, 1);
+          break;
         }
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};   // four chains instead of one long one
+        ++sn;
+        tc_fence_after();
+        // 168 registers do not hold the row and everything else: its last part is read for the maximum and again when
+        // its turn comes (P overwrites only the first half of the scores)
+        constexpr int kKept = SPLIT ? 64 : 96;
+        uint32_t v[kKept];
+        const bool diag = p.causal && (SPLIT ? 2 * j + x : j) == qt;   // keys after the query: 0 after the exponential
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};    // four chains instead of one long one
+        {
+          uint32_t t[128 - kKept];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], __uint_as_float(v[i]));
-        mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
-      }
-      const float m_new = fmaxf(m_run, mx * p.scale_log2);
-      const float alpha = fast_exp2(m_run - m_new);       // 0 for the first tile (m_run = -inf)
-      // P overwrites the buffer the previous P V product reads: that product must have completed
-      if (j >= 1 && !mbar_wait(bar(12 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, p.timeout_ns, abort_flag)) fail(j, 3);
-      float sum = 0.f;
-      float s4[4] = {0.f, 0.f, 0.f, 0.f};
-      if (ok) {
-        // keys half*64 .. +63 of this row = 64-key block `half`, eight 16-byte pieces, swizzled by the row
-        const uint32_t base = p_s + half * kHalfBytes + row * 128;
+          for (int c = kKept; c < 128; c += 32) tmem_ld_32x32b_x32(s_t + c, t + c - kKept);
 #pragma unroll
-        for (int c2 = 0; c2 < 2; ++c2) {   // pass 2, 32 scores at a time
-          uint32_t v[32];
-          tmem_ld_32x32b_x32(tmem + lane_addr + st * 128 + half * 64 + c2 * 32, v);
+          for (int c = 0; c < kKept; c += 32) tmem_ld_32x32b_x32(s_t + c, v + c);
           tmem_wait_ld();
-          if (diag) {
+          if (diag) mask_after<128 - kKept>(t, row - kKept), mask_after<kKept>(v, row);
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (half * 64 + c2 * 32 + i > row) v[i] = 0xff800000u;
-          }
+          for (int i = 0; i < 128 - kKept; i += 8)
 #pragma unroll
-          for (int qq = 0; qq < 4; ++qq) {
-            const int q = c2 * 4 + qq;       // 16-byte piece (8 keys) of this thread's 64 keys
-            uint32_t pk[4];
+            for (int c = 0; c < 4; ++c)
+              m4[c] = fmaxf(fmaxf(m4[c], __uint_as_float(t[i + 2 * c])), __uint_as_float(t[i + 2 * c + 1]));
+        }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int c = qq * 8 + 2 * i;  // index inside v
-              float e0 = fast_exp2(__uint_as_float(v[c]) * p.scale_log2 - m_new);
-              float e1 = fast_exp2(__uint_as_float(v[c + 1]) * p.scale_log2 - m_new);
-              s4[i] += e0 + e1;
-              if (F16) {
-                __half2 hh = __floats2half2_rn(e0, e1);
-                pk[i] = *reinterpret_cast<uint32_t*>(&hh);
-              } else {
-                __nv_bfloat162 bb = __floats2bfloat162_rn(e0, e1);
-                pk[i] = *reinterpret_cast<uint32_t*>(&bb);
-              }
-            }
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(base + ((q ^ (row & 7)) << 4)), "r"(pk[0]),
-                         "r"(pk[1]), "r"(pk[2]), "r"(pk[3])
-                         : "memory");
+        for (int i = 0; i < kKept; i += 8)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            m4[c] = fmaxf(fmaxf(m4[c], __uint_as_float(v[i + 2 * c])), __uint_as_float(v[i + 2 * c + 1]));
+        const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+        if (j == 0) {
+          m_run = mx;
+        } else if (__any_sync(0xffffffffu, mx > m_run + kRescaleStep)) {
+          // rare: take the new maximum and rescale what has been summed.  These scores are complete, so the products
+          // issued before them are too, and the next one waits for P.
+          const float m_new = mx > m_run + kRescaleStep ? mx : m_run;
+          const float alpha = m_new == m_run ? 1.f : fast_exp2(m_run - m_new);
+          l_run *= alpha;
+          m_run = m_new;
+#pragma unroll 1
+          for (int c = 0; c < 8; ++c) {
+            uint32_t o[16];
+            tmem_ld_32x32b_x16(o_t + x * 128 + c * 16, o);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x32b_x16(o_t + x * 128 + c * 16, o);
           }
         }
-        sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        l_run = l_run * alpha + sum;
-        m_run = m_new;
-        fence_proxy_async_smem();   // P is read by the tensor core through the async proxy
+        const float2 neg = make_float2(-m_run, -m_run);
+        float2 s2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (c * 32 >= kKept) {   // into registers that are free again
+            tmem_ld_32x32b_x32(s_t + c * 32, v + c * 32 % kKept);
+            tmem_wait_ld();
+            if (diag) mask_after<32>(v + c * 32 % kKept, row - c * 32);
+          }
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int e = c * 32 % kKept + 2 * i;
+            const float2 t = fma2(make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), scale2, neg);
+            const float2 q = make_float2(fast_exp2(t.x), fast_exp2(t.y));
+            s2[i & 1] = add2(s2[i & 1], q);
+            pk[i] = pack2<F16>(q.x, q.y);
+          }
+          tmem_st_32x32b_x16(s_t + c * 16, pk);   // P: two 16-bit values per column, over the scores this warp has read
+        }
+        tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(bar(11));        // this warp's part of P_j is in shared memory
-          mbar_arrive(bar(9 + st));    // and it has finished reading the S accumulator
-        }
-        if (j >= 1) fold_o(j - 1, alpha_prev);
-        alpha_prev = alpha;
+        if (lane == 0) mbar_arrive(p_ready(x));
+        l_run += (s2[0].x + s2[0].y) + (s2[1].x + s2[1].y);
       }
-    }
-    if (ok) fold_o(nkv - 1, alpha_prev);
-    // total row sum = the two halves' sums
-    xchg[half * 128 + row] = ok ? l_run : NAN;
-    named_barrier_sync(1, 256);
-    const float l_other = xchg[(half ^ 1) * 128 + row];
-    if (ok && l_other == l_other) {
-      const float inv = 1.f / (l_run + l_other);
+      // ---- output ----
+      const int b = it.bh / p.heads, h = it.bh - b * p.heads;
       uint8_t* orow = reinterpret_cast<uint8_t*>(p.out) +
-                      ((int64_t)(row0 + row) * p.ldo + (int64_t)h * D + half * 64) * 2;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
+                      ((int64_t)(b * p.seq + qt * BQ + row) * p.ldo + (int64_t)h * D) * 2;
+      auto store = [&](int col, const float* f) {   // 8 columns
         uint4 o;
-        uint32_t* w = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float a = acc[c * 8 + 2 * i] * inv, bb = acc[c * 8 + 2 * i + 1] * inv;
-          if (F16) {
-            __half2 hh = __floats2half2_rn(a, bb);
-            w[i] = *reinterpret_cast<uint32_t*>(&hh);
-          } else {
-            __nv_bfloat162 t = __floats2bfloat162_rn(a, bb);
-            w[i] = *reinterpret_cast<uint32_t*>(&t);
-          }
+        o.x = pack2<F16>(f[0], f[1]);
+        o.y = pack2<F16>(f[2], f[3]);
+        o.z = pack2<F16>(f[4], f[5]);
+        o.w = pack2<F16>(f[6], f[7]);
+        *reinterpret_cast<uint4*>(orow + col * 2) = o;
+      };
+      auto release = [&](int side) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(o_free(side));
+      };
+      if (!SPLIT) {
+        if (!ok) break;
+        if (!mbar_wait(o_full(x), dn & 1, p.timeout_ns, abort_flag)) {
+          stop(n, 2);
+          break;
         }
-        *reinterpret_cast<uint4*>(orow + c * 16) = o;
+        ++dn;
+        tc_fence_after();
+        const float inv = 1.f / l_run;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32b_x32(o_t + x * 128 + c * 32, o);
+          tmem_wait_ld();
+          if (c == 3) release(x);
+          float f[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(o[i]) * inv;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) store(c * 32 + q * 8, f + q * 8);
+        }
+      } else {
+        // the two sides' maxima and sums, in buffers that alternate from item to item
+        volatile float* mine = merge + (dn & 1) * 512;
+        mine[x * 256 + row] = m_run;
+        mine[x * 256 + 128 + row] = l_run;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(merge_bar);
+        if (!ok) break;
+        bool w = mbar_wait(merge_bar, dn & 1, p.timeout_ns, abort_flag);
+        w = w && mbar_wait(o_full(0), dn & 1, p.timeout_ns, abort_flag);
+        if (it.nb > 0) w = w && mbar_wait(o_full(1), bn & 1, p.timeout_ns, abort_flag);
+        if (!w) {
+          stop(n, 3);
+          break;
+        }
+        ++dn;
+        if (it.nb > 0) ++bn;
+        tc_fence_after();
+        const float ma = mine[row], la = mine[128 + row], mb = mine[256 + row], lb = mine[384 + row];
+        float fa = 1.f, fb = 0.f;
+        if (it.nb > 0) {
+          const float m = fmaxf(ma, mb);
+          fa = ma == m ? 1.f : fast_exp2(ma - m);
+          fb = mb == m ? 1.f : fast_exp2(mb - m);
+        }
+        const float inv = 1.f / (la * fa + (it.nb > 0 ? lb * fb : 0.f));
+        fa *= inv;
+        fb *= inv;
+        // side A writes the first 64 columns, side B the others
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          const int col = x * 64 + c * 16;
+          uint32_t o[16], o2[16];
+          tmem_ld_32x32b_x16(o_t + col, o);
+          if (it.nb > 0) tmem_ld_32x32b_x16(o_t + 128 + col, o2);
+          tmem_wait_ld();
+          if (c == 3) {
+            release(0);
+            if (it.nb > 0) release(1);
+          }
+          float f[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(o[i]) * fa;
+          if (it.nb > 0) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] += __uint_as_float(o2[i]) * fb;
+          }
+          store(col, f);
+          store(col + 8, f + 8);
+        }
       }
     }
   }
 
-  // ---- teardown: loads still in flight on the error path are given their barrier (bounded) ----
+  // ---- teardown ----
   __syncwarp();
-  if (*abort_flag && warp == 0 && lane == 0) {
-    volatile uint32_t never = 0;
-    for (int i = 0; i < 5; ++i) mbar_wait(bar(i), 0, 50000, &never);
-  }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 9) {
     __syncwarp();
     tmem_dealloc(tmem, 512);
   }
@@ -363,6 +617,30 @@ EncodeTiledFn attn_encode_fn() {
       (void)cudaGetLastError();
   });
   return fn;
+}
+// Whether the two sides of a CTA share out the keys of one query tile instead of taking two query tiles: if the CTA with
+// the most to do is done clearly earlier.  Time is counted in steps in which both sides do a tile of keys, plus one step
+// per item for its start and its output.  Half the chain is what counts when there are few items: 3 x 384 tokens x 5
+// heads takes 9.3 us with the keys shared out, 2 x 1024 x 12 goes from 23.8 to 15.9 us; with many items the pairs win, because
+// they load every key tile once for 256 queries instead of 128.
+bool split_keys(int batch, int seq, int heads, bool causal, int sms) {
+  const long long nq = seq / iris::attn::BQ, bh = (long long)batch * heads;
+  auto makespan = [&](bool split) {
+    const long long blocks = split ? nq : (nq + 1) / 2;
+    long long total = 0, longest = 0;
+    for (long long b = 0; b < blocks; ++b) {
+      const long long keys = !causal ? nq : split ? b + 1 : (2 * b + 2 < nq ? 2 * b + 2 : nq);
+      const long long steps = (split ? (keys + 1) / 2 : keys) + 1;
+      total += steps;
+      if (steps > longest) longest = steps;
+    }
+    const long long even = (total * bh + sms - 1) / sms;
+    // equal items: whole rounds
+    const long long rounds = (blocks * bh + sms - 1) / sms;
+    const long long t = causal ? even : rounds * longest;
+    return t > longest ? t : longest;
+  };
+  return 1.15 * makespan(true) < makespan(false);
 }
 }  // namespace
 
@@ -418,19 +696,45 @@ int iris_k_attention_fwd(const void* qkv, int64_t ld_qkv, void* out, int64_t ldo
   p.heads = heads;
   p.causal = causal ? 1 : 0;
   p.scale_log2 = 1.4426950408889634f / 11.313708498984761f;   // log2(e) / sqrt(128)
-  auto kern = dtype ? attention_fwd_kernel<true> : attention_fwd_kernel<false>;
-  static std::once_flag attr_once[2];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    snprintf(g_attn_err, sizeof(g_attn_err), "attention: no device");
+    return -3;
+  }
+  const int split = split_keys(batch, seq, heads, causal != 0, sms) ? 1 : 0;
+  auto kern = split ? (dtype ? attention_fwd_kernel<true, true> : attention_fwd_kernel<false, true>)
+                    : (dtype ? attention_fwd_kernel<true, false> : attention_fwd_kernel<false, false>);
+  static std::once_flag attr_once[4];
   cudaError_t e = cudaSuccess;
-  std::call_once(attr_once[dtype], [&]() {
+  std::call_once(attr_once[dtype * 2 + split], [&]() {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   });
   if (e != cudaSuccess) {
     snprintf(g_attn_err, sizeof(g_attn_err), "attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return -3;
   }
-  const int grid = batch * heads * (seq / BQ);
-  kern<<<grid, kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(p);
-  e = cudaGetLastError();
+  p.blocks = split ? seq / BQ : (seq / BQ + 1) / 2;
+  // Heads dealt out together: two rounds of items, the lengths of which then add up to the same for every CTA, and whose
+  // K and V (about 300 items x 256 rows x 512 bytes = 39 MB) stay in L2 until their last item.
+  p.group = (2 * sms + p.blocks - 1) / p.blocks;
+  if ((long long)batch * heads * p.blocks > 0x7fffffffLL / 2) {
+    snprintf(g_attn_err, sizeof(g_attn_err), "attention: too many query tiles");
+    return -1;
+  }
+  p.items = batch * heads * p.blocks;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.items < sms ? p.items : sms);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see grid_dependency_wait() in the kernel
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&p};
+  e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), args);
   if (e != cudaSuccess) {
     snprintf(g_attn_err, sizeof(g_attn_err), "attention: launch: %s", cudaGetErrorString(e));
     return -3;

@@ -59,3 +59,39 @@ def test_attention_large_logits_and_rejects_bad_shapes():
         attention_fwd(qkv[:500], out[:500], 1, 500, heads)       # seq not a multiple of 128
     with pytest.raises(TypeError):
         attention_fwd(qkv.float(), out, batch, seq, heads)
+
+
+@pytest.mark.parametrize("batch,seq,heads,causal,dtype", [
+    (1, 128, 5, False, torch.float16),      # one key tile: the second side of the split form has nothing to merge
+    (2, 640, 14, True, torch.bfloat16),     # 140 query tiles: split form, odd and even numbers of key tiles
+    (1, 2048, 3, False, torch.bfloat16),    # split form, a long chain
+    (3, 640, 10, True, torch.float16),      # 150 query tiles: pairs, the last tile of every head alone
+    (2, 384, 80, False, torch.bfloat16),    # pairs, several items per CTA, an incomplete last round
+    (5, 1024, 30, True, torch.bfloat16),    # pairs, several groups of heads
+])
+def test_attention_both_forms(batch, seq, heads, causal, dtype):
+    """The form in which two query tiles share their keys, and the one in which the keys of a query tile are shared out
+    and merged.  Queries grow along the keys' order, so that running maxima move by more than the rescaling step."""
+    g = torch.Generator(device="cuda").manual_seed(seq + heads)
+    t, w = batch * seq, heads * 128
+    qkv = torch.randn((t, 3 * w), generator=g, device="cuda")
+    ramp = torch.linspace(0.1, 4.0, seq, device="cuda").repeat(batch)[:, None]
+    qkv[:, w:2 * w] *= ramp                                   # later keys: larger scores
+    qkv[: t // 2, :w] *= 3.0
+    qkv = qkv.to(dtype)
+    outs = [torch.full((t, w), float("nan"), dtype=dtype, device="cuda") for _ in range(2)]
+    status = torch.zeros(16, dtype=torch.int32, device="cuda")
+    for out in outs:
+        attention_fwd(qkv, out, batch, seq, heads, causal=causal, status=status)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0, f"a wait of the kernel ran out: {status[:8].tolist()}"
+    assert torch.equal(outs[0], outs[1])
+    v_max = qkv[:, 2 * w:].float().abs().max().item()
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for b in range(batch):
+        rows = slice(b * seq, (b + 1) * seq)
+        ref = _reference(qkv[rows], 1, seq, heads, causal)
+        # every weight is rounded once (half a unit of it; the weights add up to 1), the output once more, and ex2.approx
+        # is off by 2 units in 24 bits
+        err = (outs[0][rows].float() - ref).abs().max().item()
+        assert err <= 1.05 * unit * 2 * v_max, f"batch {b}: {err}"
