@@ -22,7 +22,10 @@
 //                   most 256, which changes neither its relative rounding nor that of the fp32 sums).
 //   warp 8          TMA producer: Q tiles, and K / V tiles through a ring of five slots (no multicast)
 //   warp 9          one elected thread issues tcgen05.mma:  S = Q K^T, then O += P V (P from tensor memory, V as an
-//                   MN-major operand: V[key][d] is read as stored), alternating between the sides
+//                   MN-major operand: V[key][d] is read as stored), alternating between the sides; the first half of a
+//                   product starts when the first half of P is there
+// What bounds it: the pair form the GPU's power limit (1.17 PFLOP/s without a mask from a rest, less in a long run), the split
+// form the chain scores -> softmax -> product of one side, about 3000 cycles per tile.
 // Before: one 128-row tile per CTA, two threads per row reading the scores twice, P through shared memory, O folded
 // through registers after every tile.  8 x 2048 tokens x 32 heads, causal, bf16: 668 -> 333 us back to back (power-limited), 649 -> 280 us from a rest.
 //
@@ -63,6 +66,11 @@ static_assert(kSmemBytes <= 227 * 1024, "shared-memory budget");
 // limit of 65504.
 constexpr float kRescaleStep = 8.f;
 
+// The split form, in which the softmax of a tile is part of the chain that sets the time, makes one in so many pairs of
+// exponentials on the FMA units instead of the special-function unit (1 x 4096 x 4 heads causal: 37.3 -> 33.4 us; every
+// third 33.5).  The pair form gains nothing from it (281 -> 285 us).
+constexpr int kPolyEvery = 4;
+
 enum Site : uint32_t { kSiteLoad = 90, kSiteMma = 91, kSiteSoftmax = 92 };
 
 // 2^x on the special-function unit (ex2.approx: 2 ulp, 2^-inf = 0), which is what bounds the softmax warps.
@@ -70,6 +78,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 // Two fp32 operations in one instruction.
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -87,6 +100,33 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
       : "=f"(d.x), "=f"(d.y)
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\t"
+      "mov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+// 2^t on the FMA units, for a share of the exponentials (see kPolyEvery).  t = k + f with k the nearest integer, 2^f from a
+// polynomial of degree 5 with value 1 at 0, fitted here for the smallest largest relative error on [-1/2, 1/2]: 9.1e-08 in
+// exact arithmetic, 1.7e-7 evaluated in fp32 (ex2.approx: 2.4e-7).  t below -126 gives 2^-126 instead of 0, a NaN stays one.
+__device__ __forceinline__ float2 poly_exp2(float2 t) {
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(t.x));   // -126
+  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(t.y));
+  const float kMagic = 12582912.f;   // 1.5 * 2^23: the sum's last bits are the integer part
+  const float2 r = add2(t, make_float2(kMagic, kMagic));
+  const float2 k = add2(r, make_float2(-kMagic, -kMagic));
+  const float2 f = fma2(k, make_float2(-1.f, -1.f), t);
+  auto both = [](float c) { return make_float2(c, c); };
+  float2 q = fma2(both(1.326472731e-03f), f, both(9.671512991e-03f));
+  q = fma2(q, f, both(5.550733581e-02f));
+  q = fma2(q, f, both(2.402224243e-01f));
+  q = fma2(q, f, both(6.931470037e-01f));
+  q = fma2(q, f, both(1.f));
+  return mul2(q, make_float2(__uint_as_float((__float_as_uint(r.x) << 23) + 0x3f800000u),
+                             __uint_as_float((__float_as_uint(r.y) << 23) + 0x3f800000u)));
 }
 template <bool F16>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
@@ -166,9 +206,10 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
   auto q_full = [&](int x) { return bar0 + 8u * (0 + x); };
   auto q_empty = [&](int x) { return bar0 + 8u * (2 + x); };
   auto s_full = [&](int x) { return bar0 + 8u * (4 + x); };    // scores complete (and everything issued before them)
-  auto p_ready = [&](int x) { return bar0 + 8u * (6 + x); };   // P in tensor memory, scores read, O rescaled
+  auto p_half = [&](int x) { return bar0 + 8u * (6 + x); };    // P of the first 64 keys in tensor memory, O rescaled
   auto o_full = [&](int x) { return bar0 + 8u * (8 + x); };    // last product of the item complete
   auto o_free = [&](int x) { return bar0 + 8u * (10 + x); };   // O has been read
+  auto p_ready = [&](int x) { return bar0 + 8u * (14 + x); };  // all of P in tensor memory, scores read
   const uint32_t merge_bar = bar0 + 8u * 12;                   // split: both sides' maxima and sums are in shared memory
   const uint32_t drain_bar = bar0 + 8u * 13;
   auto kv_full = [&](int s) { return bar0 + 8u * (16 + s); };
@@ -186,7 +227,8 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
       mbar_init(q_full(x), 1);
       mbar_init(q_empty(x), 1);
       mbar_init(s_full(x), 1);
-      mbar_init(p_ready(x), 4);                  // one arrival per softmax warp of the side
+      mbar_init(p_half(x), 4);                   // one arrival per softmax warp of the side
+      mbar_init(p_ready(x), 4);
       mbar_init(o_full(x), 1);
       mbar_init(o_free(x), SPLIT ? 8 : 4);     // split: both sides read both outputs
     }
@@ -351,18 +393,27 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
             const uint32_t pos = base + pos_v(it, key_tile(x, j));
             const int s = pos % kSlots;
             if (!mbar_wait(kv_full(s), (pos / kSlots) & 1, p.timeout_ns, abort_flag) ||
-                !mbar_wait(p_ready(x), sn[x] & 1, p.timeout_ns, abort_flag)) {
+                !mbar_wait(p_half(x), sn[x] & 1, p.timeout_ns, abort_flag)) {
               stop(3);
+              break;
+            }
+            tc_fence_after();
+            // 16 keys = two groups of 8 rows (1024 bytes apart); the second 64 columns of d are one half tile further on
+            const uint64_t vd = umma_desc_mn_sw128(ring + s * kTileBytes, kHalfBytes, 1024);
+            auto product = [&](int k0) {   // 64 keys
+#pragma unroll
+              for (int kk = k0; kk < k0 + BKV / 32; ++kk)
+                umma_f16_ts(tmem + 256 + x * 128, tmem + x * 128 + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv,
+                            (j > 0 || kk > 0) ? 1u : 0u);
+            };
+            product(0);   // runs while the other half's exponentials are made
+            if (!mbar_wait(p_ready(x), sn[x] & 1, p.timeout_ns, abort_flag)) {
+              stop(4);
               break;
             }
             ++sn[x];
             tc_fence_after();
-            // 16 keys = two groups of 8 rows (1024 bytes apart); the second 64 columns of d are one half tile further on
-            const uint64_t vd = umma_desc_mn_sw128(ring + s * kTileBytes, kHalfBytes, 1024);
-#pragma unroll
-            for (int kk = 0; kk < BKV / 16; ++kk)
-              umma_f16_ts(tmem + 256 + x * 128, tmem + x * 128 + kk * 8, vd + kk * (16 * 128 >> 4), idesc_pv,
-                          (j > 0 || kk > 0) ? 1u : 0u);
+            product(BKV / 32);
             if (last_use(it, x, j)) umma_commit(kv_empty(s));
             if (j + 1 < n) {
               scores(it, base, x, j + 1);
@@ -437,13 +488,13 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
           for (int i = 0; i < 128 - kKept; i += 8)
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-              m4[c] = fmaxf(fmaxf(m4[c], __uint_as_float(t[i + 2 * c])), __uint_as_float(t[i + 2 * c + 1]));
+              m4[c] = max3(m4[c], __uint_as_float(t[i + 2 * c]), __uint_as_float(t[i + 2 * c + 1]));
         }
 #pragma unroll
         for (int i = 0; i < kKept; i += 8)
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-            m4[c] = fmaxf(fmaxf(m4[c], __uint_as_float(v[i + 2 * c])), __uint_as_float(v[i + 2 * c + 1]));
+            m4[c] = max3(m4[c], __uint_as_float(v[i + 2 * c]), __uint_as_float(v[i + 2 * c + 1]));
         const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
         if (j == 0) {
           m_run = mx;
@@ -478,11 +529,18 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
           for (int i = 0; i < 16; ++i) {
             const int e = c * 32 % kKept + 2 * i;
             const float2 t = fma2(make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), scale2, neg);
-            const float2 q = make_float2(fast_exp2(t.x), fast_exp2(t.y));
+            const float2 q = SPLIT && i % kPolyEvery == kPolyEvery - 1 ? poly_exp2(t)
+                                                              : make_float2(fast_exp2(t.x), fast_exp2(t.y));
             s2[i & 1] = add2(s2[i & 1], q);
             pk[i] = pack2<F16>(q.x, q.y);
           }
           tmem_st_32x32b_x16(s_t + c * 16, pk);   // P: two 16-bit values per column, over the scores this warp has read
+          if (c == 1) {
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_half(x));
+          }
         }
         tmem_wait_st();
         tc_fence_before();

@@ -95,3 +95,29 @@ def test_attention_both_forms(batch, seq, heads, causal, dtype):
         # is off by 2 units in 24 bits
         err = (outs[0][rows].float() - ref).abs().max().item()
         assert err <= 1.05 * unit * 2 * v_max, f"batch {b}: {err}"
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 1), (2, 40)])   # keys of a query tile shared out; pairs of query tiles
+@pytest.mark.parametrize("key", [0, 5, 6, 7, 130, 255])
+def test_attention_keeps_nan_and_infinity_of_a_key(batch, heads, key):
+    """A NaN in one key reaches every query that may see it, whichever unit makes its exponential, and no other; a key whose
+    scores are minus infinity weighs nothing."""
+    g = torch.Generator(device="cuda").manual_seed(key)
+    seq, w = 256, heads * 128
+    qkv = torch.randn((batch * seq, 3 * w), generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.empty((batch * seq, w), dtype=torch.bfloat16, device="cuda")
+    bad = qkv.clone()
+    bad[key, w:w + 128] = float("nan")                        # batch 0, head 0
+    attention_fwd(bad, out, batch, seq, heads, causal=True)
+    nan = torch.isnan(out.float())
+    want = torch.zeros_like(nan)
+    want[key:seq, :128] = True
+    assert torch.equal(nan, want)
+    if key > 0:
+        bad = qkv.clone()
+        bad[:, :128] = bad[:, :128].abs() + 0.1               # head 0: positive queries, a key of minus infinity
+        bad[key, w:w + 128] = float("-inf")
+        attention_fwd(bad, out, batch, seq, heads, causal=True)
+        ref = _reference(bad[:seq], 1, seq, heads, True)[:, :128]
+        # as in test_attention_both_forms
+        assert (out[:seq, :128].float() - ref).abs().max().item() <= 1.05 * 2.0 ** -7 * bad[:, 2 * w:].float().abs().max().item()
