@@ -20,6 +20,7 @@ shapes, or with ``attention="sdpa"``) calls ``torch.nn.functional.scaled_dot_pro
 """
 from __future__ import annotations
 
+import os
 from dataclasses import dataclass
 from typing import List, Sequence, Union
 
@@ -120,6 +121,8 @@ class TPDecoder:
         self.own_attention = attention == "iris" and cfg.head_dim == A.HEAD_DIM and cfg.seq % 128 == 0
         self.ts = T // W
         nl = len(self.ctxs)
+        # one rank: the gate / up projection applies the SwiGLU on its way out (its own kernel otherwise)
+        self.fused_swiglu = W == 1 and "IRIS_STREAM_K" not in os.environ
         self.attn = [torch.empty((T, H // W), dtype=torch.bfloat16, device=dev) for _ in range(nl)]
         self.h = [torch.empty((T, I // W), dtype=torch.bfloat16, device=dev) for _ in range(nl)]
         self.layers = []
@@ -131,7 +134,8 @@ class TPDecoder:
                 "w": sh,
                 "qkv": G.all_gather_gemm(self.ctxs, T, [s["wqkv"] for s in sh], ag_slices=ag_slices),
                 "o": row_parallel(self.attn, [s["wo"] for s in sh]),
-                "gu": G.all_gather_gemm(self.ctxs, T, [s["wgu"] for s in sh], ag_slices=ag_slices),
+                "gu": G.all_gather_gemm(self.ctxs, T, [s["wgu"] for s in sh], ag_slices=ag_slices,
+                                        **(dict(swiglu=True, out=self.h) if self.fused_swiglu else {})),
                 "down": row_parallel(self.h, [s["wd"] for s in sh]),
             }
             self.layers.append(ops)
@@ -173,12 +177,12 @@ class TPDecoder:
             tick("gu_ag_gemm")
             gu = ops["gu"]()
             tick("swiglu")
-            for l in range(nl):
+            for l in range(nl if not self.fused_swiglu else 0):
                 E.swiglu(gu[l], self.h[l])
             tick("down_gemm_ar")
             d = ops["down"]()
             pending = [d[l] if self.scatter else d[l][self.rows(l)] for l in range(nl)]
-            n += 4 + 4 * nl     # 4 fused GEMMs; per rank: norm, attention, add+norm, SwiGLU
+            n += 4 + (3 if self.fused_swiglu else 4) * nl   # 4 fused GEMMs; per rank: norm, attention, add+norm, SwiGLU
         tick("norm")
         for l in range(nl):
             E.residual_add(x_shards[l], pending[l])

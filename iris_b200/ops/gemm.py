@@ -77,7 +77,7 @@ def _lib():
         operands = [ptr, i64, ptr, i64, ptr, i64, i32, i32, i32, i32, i32, ptr, ctypes.c_uint64, i32, i32, i32, i32]
         lib.iris_gemm_local_last_error.restype = ctypes.c_char_p
         lib.iris_gemm_local_create.restype = ptr
-        lib.iris_gemm_local_create.argtypes = operands
+        lib.iris_gemm_local_create.argtypes = operands + [i32]
         lib.iris_gemm_local.argtypes = operands + [ptr]
         lib.iris_gemm_local_launch.argtypes = [ptr, ptr]
         lib.iris_gemm_local_destroy.argtypes = [ptr]
@@ -147,6 +147,9 @@ class FusedGemm:
             bytes on a heap bound to an NVLS multicast object: the switch delivers it to every rank).  ``None``:
             ``DEFAULT_PUSH_KIND``.
 
+        swiglu: (one rank, mode ``"store"``, bf16 / fp16) ``bt`` holds the rows of a gate and those of a linear
+            projection, one block after the other, and the output is ``silu(a @ gate.T) * (a @ linear.T)``, half as wide.
+
     The element type is taken from ``bt``: bf16 or fp16 (fp32 accumulation) for every mode; float32 (multiplied as
     tf32, fp32 accumulation) and int8 (32-bit integer accumulation, the low 8 bits of the sum as the result, which is
     what the reference's kernel stores when it casts its int32 accumulator to the output type) for mode ``"store"``:
@@ -162,12 +165,12 @@ class FusedGemm:
                  cta_group: Optional[int] = None, trace: bool = False, stream_k: Optional[bool] = None,
                  push: Optional[bool] = None, ksplit: Optional[int] = None, nvls: Optional[bool] = None,
                  reduce_scatter: bool = False, bn: Optional[int] = None, tail_split: Optional[bool] = None,
-                 push_kind: Optional[str] = None, bcast: bool = False):
+                 push_kind: Optional[str] = None, bcast: bool = False, swiglu: bool = False):
         self._ctor = (ctxs, a, bt, mode, dict(
             M=M, store_all=store_all, c_cols=c_cols, col_off_per_rank=col_off_per_rank, out=out, ag=ag,
             ag_slices=ag_slices, ctas_per_rank=ctas_per_rank, group_m=group_m, timeout_ms=timeout_ms,
             cta_group=cta_group, trace=trace, stream_k=stream_k, push=push, ksplit=ksplit, nvls=nvls,
-            reduce_scatter=reduce_scatter, bn=bn, tail_split=tail_split, push_kind=push_kind, bcast=bcast))
+            reduce_scatter=reduce_scatter, bn=bn, tail_split=tail_split, push_kind=push_kind, bcast=bcast, swiglu=swiglu))
         self.ctxs: List[Iris] = [ctxs] if isinstance(ctxs, Iris) else list(ctxs)
         c0 = self.ctxs[0]
         if c0.backend != "cuda":
@@ -211,6 +214,12 @@ class FusedGemm:
             x is None for x in (ctas_per_rank, group_m, cta_group, stream_k, push, ksplit, bn, tail_split, push_kind)))
         if self.local:
             stream_k = False
+        self.swiglu = bool(swiglu)
+        if self.swiglu:
+            if not (self.local and mode == "store" and self.N % 2 == 0 and self.dtype in (torch.bfloat16, torch.float16)):
+                raise ValueError("swiglu=True: one rank, mode 'store', 16-bit elements, an even number of rows of B and no "
+                                 "explicit schedule")
+            c_cols = self.N // 2
         # tile shape, persistent grid, schedule, flag count and buffer layout: a pure function of the problem
         pl = plan_gemm(self.M, self.N, self.K, self.world, self.num_local, mode, sms, ag=self.ag, cta_group=cta_group,
                        ctas_per_rank=ctas_per_rank, group_m=group_m, stream_k=stream_k, push=push, ksplit=ksplit,
@@ -333,16 +342,19 @@ class FusedGemm:
         d.mc_base = mc if (self.nvls or pk == "multimem") else 0
         self.ag_slices = int(ag_slices)
         lib = _lib()
-        self._plan = lib.iris_gemm_plan_create(ctypes.byref(d))
-        if not self._plan:
-            raise RuntimeError("fused GEMM plan: " + lib.iris_gemm_last_error().decode())
-        self.ctas_per_rank = lib.iris_gemm_plan_ctas_per_rank(self._plan)  # what fits on the device
+        if not self.swiglu:
+            self._plan = lib.iris_gemm_plan_create(ctypes.byref(d))
+            if not self._plan:
+                raise RuntimeError("fused GEMM plan: " + lib.iris_gemm_last_error().decode())
+            self.ctas_per_rank = lib.iris_gemm_plan_ctas_per_rank(self._plan)  # what fits on the device
         if self.local:   # the fused plan has vetted the arguments; what runs is the one-rank kernel
-            lib.iris_gemm_plan_destroy(self._plan)
+            if not self.swiglu:
+                lib.iris_gemm_plan_destroy(self._plan)
             a0, b0, o0 = a_use[0], bt[0], self.out[0]
             self._plan = lib.iris_gemm_local_create(
-                a0.data_ptr(), a0.stride(0), b0.data_ptr(), b0.stride(0), o0.data_ptr(), o0.stride(0), self.M, self.N,
-                self.K, d.dtype, c0.gpu_id, c0.status.data_ptr(), d.timeout_ns, -1, 0, 0, 0)
+                a0.data_ptr(), a0.stride(0), b0.data_ptr(), b0.stride(0), o0.data_ptr(), o0.stride(0), self.M,
+                self.N // 2 if self.swiglu else self.N, self.K, d.dtype, c0.gpu_id, c0.status.data_ptr(), d.timeout_ns, -1, 0,
+                0, 0, int(self.swiglu))
             if not self._plan:
                 raise RuntimeError("GEMM plan: " + lib.iris_gemm_local_last_error().decode())
             info = (ctypes.c_int * 6)()

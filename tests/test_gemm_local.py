@@ -136,3 +136,38 @@ def test_choice_matches_and_repeats(m, n, k, dtype):
         graph.reset()
         op.close()
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,inter,k,dtype", [(1, 8, 64, "bf16"), (128, 1376, 512, "bf16"), (129, 200, 264, "fp16"),
+                                             (700, 2744, 1032, "bf16"), (2048, 1024, 512, "fp16")])
+def test_gate_and_linear_projection_in_one(m, inter, k, dtype):
+    """``swiglu=True`` against silu(a gate^T) * (a linear^T) in float64.  Off by the output's rounding, by the fp32 sums'
+    K * 2^-24 of their magnitudes (times what either factor scales them by; silu' <= 1.1), and by 2^-20 of the value for
+    the fast exponential and division."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import iris_b200 as iris
+    from iris_b200.ops import gemm as G
+    a = _operand((m, k), dtype, 1)
+    bt = (_operand((2 * inter, k), dtype, 2).float() / k ** 0.5).to(TYPES[dtype])
+    frame = torch.full((m, inter + 16), 3, dtype=TYPES[dtype], device="cuda")
+    ctx = iris.iris(128 << 20)
+    op = G.all_gather_gemm(ctx, (m + 127) // 128 * 128, [bt], swiglu=True)
+    op.a_full[0][:m].copy_(a)
+    got = op()[0][:m]
+    op.check()
+    own = G.FusedGemm(ctx, [a], [bt], "store", out=[frame[:, 8:8 + inter]], swiglu=True)
+    own()
+    own.check()
+    assert got.shape == (m, inter) and torch.equal(frame[:, 8:8 + inter], got)
+    assert bool((frame[:, :8] == 3).all()) and bool((frame[:, 8 + inter:] == 3).all())
+    g, u = a.double() @ bt[:inter].double().t(), a.double() @ bt[inter:].double().t()
+    sg, su = (a.double().abs() @ b.double().abs().t() for b in (bt[:inter], bt[inter:]))
+    exact = g * torch.sigmoid(g) * u
+    unit = 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
+    bound = (unit + 2.0 ** -20) * exact.abs() + k * 2.0 ** -24 * (1.1 * sg * u.abs() + g.abs() * su) + 2.0 ** -24
+    assert bool(((got.double() - exact).abs() <= 1.01 * bound).all())
+    with pytest.raises(ValueError):
+        G.FusedGemm(ctx, [a], [bt], "store", swiglu=True, bn=64)
+    op.close(), own.close(), ctx.close()
