@@ -190,8 +190,9 @@ class MessagePassing:
         if roles == 0:
             return
         lib = _native.kernels()
-        lib.iris_k_message_passing.argtypes = [ctypes.c_void_p] + [ctypes.c_uint64] * 6 + [ctypes.c_int] * 5 + \
-            [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p]
+        if lib.iris_k_message_passing.argtypes is None:
+            lib.iris_k_message_passing.argtypes = [ctypes.c_void_p] + [ctypes.c_uint64] * 6 + [ctypes.c_int] * 5 + \
+                [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p]
         parts = self.parts   # with roles == 3 the launcher lowers the block count to what is resident at once
         rc = lib.iris_k_message_passing(
             _hb(ctx), ctx.offset_of(self.src), ctx.offset_of(self.dst), ctx.offset_of(self.out),
