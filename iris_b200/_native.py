@@ -100,7 +100,23 @@ def rt_check(rc: int, what: str = "") -> None:
 
 
 def kernels() -> ctypes.CDLL:
-    return _load("kernels")
+    return _cache.get("kernels") or _load("kernels")
+
+
+def typed(fn, argtypes, restype=c_int):
+    """``fn`` with its argument types set, once (setting them costs as much as a short call)."""
+    if fn.argtypes is None:
+        fn.argtypes, fn.restype = argtypes, restype
+    return fn
+
+
+def current_stream(device_index) -> int:
+    """The handle of PyTorch's current stream on CUDA device ``device_index`` (``tensor.get_device()``): what
+    ``torch.cuda.current_stream(...).cuda_stream`` gives, without making the stream object (2 us, as much as a launch)."""
+    import torch
+    if device_index is None or device_index < 0:
+        raise ValueError("expected a tensor or context on a CUDA device")
+    return torch._C._cuda_getCurrentRawStream(device_index)
 
 
 def kernels_available() -> bool:

@@ -15,6 +15,8 @@ from .. import _native
 
 HEAD_DIM = 128
 _DT = {torch.bfloat16: 0, torch.float16: 1}
+_ARGTYPES = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+             ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]
 
 
 def attention_fwd(qkv: torch.Tensor, out: torch.Tensor, batch: int, seq: int, heads: int, causal: bool = True,
@@ -34,15 +36,11 @@ def attention_fwd(qkv: torch.Tensor, out: torch.Tensor, batch: int, seq: int, he
         raise ValueError(f"expected qkv [{batch * seq}, {3 * heads * HEAD_DIM}] and out [{batch * seq}, "
                          f"{heads * HEAD_DIM}], got {tuple(qkv.shape)} and {tuple(out.shape)}")
     lib = _native.kernels()
-    fn = lib.iris_k_attention_fwd
-    fn.restype = ctypes.c_int
-    fn.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_int,
-                   ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]
-    lib.iris_attention_last_error.restype = ctypes.c_char_p
-    st = torch.cuda.current_stream(qkv.device).cuda_stream if stream is None else stream
+    fn = _native.typed(lib.iris_k_attention_fwd, _ARGTYPES)
+    st = _native.current_stream(qkv.get_device()) if stream is None else stream
     rc = fn(qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), batch, seq, heads, int(bool(causal)),
-            _DT[qkv.dtype], ctypes.c_void_p(status.data_ptr() if status is not None else 0), int(timeout_ms * 1e6),
-            ctypes.c_void_p(st))
+            _DT[qkv.dtype], status.data_ptr() if status is not None else 0, int(timeout_ms * 1e6), st)
     if rc != 0:
+        lib.iris_attention_last_error.restype = ctypes.c_char_p
         raise RuntimeError(lib.iris_attention_last_error().decode() or f"attention launch failed ({rc})")
     return out

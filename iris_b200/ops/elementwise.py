@@ -10,8 +10,11 @@ import torch
 from .. import _native
 
 
+_P, _L, _I, _F = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float
+
+
 def _st(t, stream):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream if stream is None else stream)
+    return _native.current_stream(t.get_device()) if stream is None else stream
 
 
 def _check2d(t, name):
@@ -23,10 +26,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float
     """``out = x * rsqrt(mean(x^2, -1) + eps) * weight`` row by row; ``out`` may be a row block of a larger matrix."""
     _check2d(x, "x"), _check2d(out, "out")
     lib = _native.kernels()
-    lib.iris_k_rmsnorm_bf16.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p,
-                                        ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_float, ctypes.c_void_p]
-    rc = lib.iris_k_rmsnorm_bf16(x.data_ptr(), x.stride(0), weight.data_ptr(), out.data_ptr(), out.stride(0),
-                                 x.shape[0], x.shape[1], eps, _st(x, stream))
+    fn = _native.typed(lib.iris_k_rmsnorm_bf16, [_P, _L, _P, _P, _L, _I, _I, _F, _P])
+    rc = fn(x.data_ptr(), x.stride(0), weight.data_ptr(), out.data_ptr(), out.stride(0), x.shape[0], x.shape[1], eps,
+            _st(x, stream))
     if rc:
         raise RuntimeError(f"rmsnorm launch failed ({rc})")
     return out
@@ -39,10 +41,9 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, stream=None) -> torch.Tenso
     if gate_up.shape[1] != 2 * inter:
         raise ValueError("gate_up must have twice the columns of out")
     lib = _native.kernels()
-    lib.iris_k_swiglu_bf16.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int,
-                                       ctypes.c_int, ctypes.c_void_p]
-    rc = lib.iris_k_swiglu_bf16(gate_up.data_ptr(), gate_up.stride(0), out.data_ptr(), out.stride(0), out.shape[0],
-                                inter, _st(out, stream))
+    fn = _native.typed(lib.iris_k_swiglu_bf16, [_P, _L, _P, _L, _I, _I, _P])
+    rc = fn(gate_up.data_ptr(), gate_up.stride(0), out.data_ptr(), out.stride(0), out.shape[0], inter,
+            _st(out, stream))
     if rc:
         raise RuntimeError(f"swiglu launch failed ({rc})")
     return out
@@ -52,10 +53,8 @@ def residual_add(x: torch.Tensor, y: torch.Tensor, stream=None) -> torch.Tensor:
     """``x += y`` in place."""
     _check2d(x, "x"), _check2d(y, "y")
     lib = _native.kernels()
-    lib.iris_k_residual_add_bf16.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64,
-                                             ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
-    rc = lib.iris_k_residual_add_bf16(x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), x.shape[0], x.shape[1],
-                                      _st(x, stream))
+    fn = _native.typed(lib.iris_k_residual_add_bf16, [_P, _L, _P, _L, _I, _I, _P])
+    rc = fn(x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), x.shape[0], x.shape[1], _st(x, stream))
     if rc:
         raise RuntimeError(f"residual_add launch failed ({rc})")
     return x
@@ -67,11 +66,9 @@ def add_rmsnorm(x: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, out: tor
     of one sub-block fused with the norm that opens the next.  ``out`` may be a row block of a larger matrix."""
     _check2d(x, "x"), _check2d(y, "y"), _check2d(out, "out")
     lib = _native.kernels()
-    lib.iris_k_add_rmsnorm_bf16.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64,
-                                            ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int,
-                                            ctypes.c_int, ctypes.c_float, ctypes.c_void_p]
-    rc = lib.iris_k_add_rmsnorm_bf16(x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), weight.data_ptr(),
-                                     out.data_ptr(), out.stride(0), x.shape[0], x.shape[1], eps, _st(x, stream))
+    fn = _native.typed(lib.iris_k_add_rmsnorm_bf16, [_P, _L, _P, _L, _P, _P, _L, _I, _I, _F, _P])
+    rc = fn(x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), weight.data_ptr(), out.data_ptr(), out.stride(0),
+            x.shape[0], x.shape[1], eps, _st(x, stream))
     if rc == -3:     # row too long for the register-resident kernel
         residual_add(x, y, stream)
         return rmsnorm(x, weight, out, eps, stream)

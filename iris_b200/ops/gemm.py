@@ -96,9 +96,10 @@ def _check_operand(t: torch.Tensor, name: str, dtype: Optional[torch.dtype] = No
         raise TypeError(f"{name} must be bfloat16, float16, float32 or int8, got {t.dtype}")
     if dtype is not None and t.dtype != dtype:
         raise TypeError(f"{name} is {t.dtype}, the other operands are {dtype}")
-    if t.dim() != 2 or t.stride(1) != 1:
+    stride = t.stride()
+    if len(stride) != 2 or stride[1] != 1:
         raise ValueError(f"{name} must be 2-D with a contiguous last dimension (K-major)")
-    if t.data_ptr() % 16 or (t.stride(0) * t.element_size()) % 16:
+    if t.data_ptr() % 16 or (stride[0] * t.element_size()) % 16:
         raise ValueError(f"{name}: base address and row pitch must be multiples of 16 bytes")
 
 
@@ -370,10 +371,10 @@ class FusedGemm:
     # every rank of a real multi-process world must call this the same number of times
     def __call__(self, stream=None) -> List[torch.Tensor]:
         c0 = self.ctxs[0]
-        st = torch.cuda.current_stream(c0.device).cuda_stream if stream is None else stream
+        st = _native.current_stream(c0.gpu_id) if stream is None else stream
         if self.local:
             self.calls += 1
-            if _lib().iris_gemm_local_launch(self._plan, ctypes.c_void_p(st)) != 0:
+            if _lib().iris_gemm_local_launch(self._plan, st) != 0:
                 raise RuntimeError("GEMM launch: " + _lib().iris_gemm_local_last_error().decode())
             self.launches += 1
             return self.out
@@ -537,6 +538,17 @@ def all_gather_gemm(ctxs, M: int, bt, **kw) -> FusedGemm:
 
 
 _private_ctx = {}
+_streams = {}
+
+
+def _stream_object(device: int, raw: int) -> "torch.cuda.Stream":
+    """The stream object of a raw handle that is current on ``device``; making one costs 2 us, and programs have few."""
+    s = _streams.get((device, raw))
+    if s is None:
+        if len(_streams) >= 64:
+            _streams.clear()
+        s = _streams[(device, raw)] = torch.cuda.current_stream(device)
+    return s
 
 
 def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
@@ -553,20 +565,22 @@ def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
     bt = as_kmajor_bt(bt)
     n = bt.shape[0]
     if out is None:
-        out = torch.empty((a.shape[0], n), dtype=a.dtype, device=dev)
+        out = a.new_empty((a.shape[0], n))
     if cta_group is None and bn is None and tail_split is None and "IRIS_STREAM_K" not in os.environ:
         _check_operand(bt, "B")
         _check_operand(a, "A", bt.dtype)
-        if a.shape[1] != bt.shape[1]:
-            raise ValueError(f"K mismatch: A has {a.shape[1]}, B has {bt.shape[1]}")
+        m, k = a.shape
+        if k != bt.shape[1]:
+            raise ValueError(f"K mismatch: A has {k}, B has {bt.shape[1]}")
         _check_operand(out, "output", bt.dtype)
-        stream = torch.cuda.current_stream(dev)
+        device = a.get_device()
+        raw = _native.current_stream(device)
         lib = _lib()
-        rc = lib.iris_gemm_local(a.data_ptr(), a.stride(0), bt.data_ptr(), bt.stride(0), out.data_ptr(), out.stride(0),
-                                 a.shape[0], n, a.shape[1], DTYPES[_TORCH_DTYPES[bt.dtype]], dev.index or 0,
-                                 ctx.status.data_ptr(), 2000000000, -1, 0, 0, 0, stream.cuda_stream)
+        rc = lib.iris_gemm_local(a.data_ptr(), a.stride(0), bt.data_ptr(), bt.stride(0), out.data_ptr(), out.stride(0), m, n, k,
+                                 DTYPES[_TORCH_DTYPES[bt.dtype]], device, ctx.status_ptr(), 2000000000, -1, 0, 0, 0, raw)
         if rc != 0:
             raise RuntimeError("GEMM: " + lib.iris_gemm_local_last_error().decode())
+        stream = _stream_object(device, raw)
         for t in (a, bt, out):   # the caller may let go of them, whatever stream they come from
             t.record_stream(stream)
         return out

@@ -20,7 +20,7 @@ def default_grid(ctx, per_sm: int = 4) -> int:
 
 
 def _stream(ctx, stream):
-    return ctypes.c_void_p(torch.cuda.current_stream(ctx.device).cuda_stream if stream is None else stream)
+    return ctypes.c_void_p(_native.current_stream(ctx.device.index) if stream is None else stream)
 
 
 def _hb(ctx):
@@ -190,11 +190,10 @@ class MessagePassing:
         if roles == 0:
             return
         lib = _native.kernels()
-        if lib.iris_k_message_passing.argtypes is None:
-            lib.iris_k_message_passing.argtypes = [ctypes.c_void_p] + [ctypes.c_uint64] * 6 + [ctypes.c_int] * 5 + \
-                [ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p]
+        fn = _native.typed(lib.iris_k_message_passing, [ctypes.c_void_p] + [ctypes.c_uint64] * 6 + [ctypes.c_int] * 5 + [
+            ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p])
         parts = self.parts   # with roles == 3 the launcher lowers the block count to what is resident at once
-        rc = lib.iris_k_message_passing(
+        rc = fn(
             _hb(ctx), ctx.offset_of(self.src), ctx.offset_of(self.dst), ctx.offset_of(self.out),
             ctx.offset_of(self.flags), ctx.offset_of(ctx.status), self.chunk_bytes, self.nchunks, self.producer,
             self.consumer, roles, int(use_put), 0 if self.device_epoch else self.epoch, self.timeout_ns, block, parts,
