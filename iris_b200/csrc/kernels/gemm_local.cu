@@ -23,7 +23,7 @@
 // and the GPU's power limit (8192 x 14336 x 4096 back to back: 761 -> 703 us, 1.37 PFLOP/s; int8 8192 x 3584 x 14336: 347 ->
 // 297 us; fp32 2048 x 4096 x 4096: 129 -> 110 us).
 //
-// Roles (192 threads, one CTA per SM): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue.  The producer starts
+// Roles (320 threads, one CTA per SM): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 epilogue.  The producer starts
 // before the block's set-up barrier (it needs only the ring barriers, which it initialises itself).
 //
 // Every wait on an mbarrier is bounded by timeout_ns: on expiry the CTA records a status, its roles leave their loops,
@@ -61,9 +61,10 @@ constexpr int kMaxCols = 256;
 constexpr int kRowsBytes = kRows * 128;  // one stage of the 128-row operand: 128 bytes of K per row
 constexpr int kMaxStages = 12;
 constexpr int kMaxCluster = 8;         // portable cluster size
-constexpr int kThreads = 192;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kBarBytes = 1024;        // barriers and the small shared words, in front of the ring
-constexpr int kStagingBytes = 2 * kRows * 128;   // two epilogue buffers of 128 rows x 128 bytes
+constexpr int kStagingBytes = kEpiWarps * 32 * 128;   // 32 rows x 128 bytes for every epilogue warp
 constexpr int kSmemMax = 227 * 1024;
 // Never less than this much shared memory: two CTAs on one SM would wait for one another's tensor memory.
 constexpr int kSmemMin = 116 * 1024;
@@ -175,7 +176,6 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
   volatile uint32_t* tmem_slot = words;
   volatile uint32_t* abort_flag = words + 1;
   volatile uint32_t* never = words + 2;
-  volatile uint32_t* verdict = words + 3;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // uniform over the warp
   const int split = p.split;
@@ -233,12 +233,11 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full_bar(b), 1);
-      mbar_init(acc_empty_bar(b), 4 * CG);   // one arrival per epilogue warp of every CTA of the tile
+      mbar_init(acc_empty_bar(b), kEpiWarps * CG);   // one arrival per epilogue warp of every CTA of the tile
     }
-    mbar_init(recv_bar, 4 * (split - 1) > 0 ? 4 * (split - 1) : 1);   // one arrival per sending warp
+    mbar_init(recv_bar, split > 1 ? kEpiWarps * (split - 1) : 1);   // one arrival per sending warp
     *abort_flag = 0;
     *never = 0;
-    *verdict = 1;
     mbar_fence_init();
     place(tile);
     if (CG == 1) {
@@ -295,12 +294,13 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       const uint32_t idesc = ET == kTf32   ? umma_idesc_tf32(TM, p.tn)
                              : ET == kInt8 ? umma_idesc_s8(TM, p.tn)
                                            : umma_idesc_f16(TM, p.tn, ET == kBf16);
+      const uint32_t own0 = CG == 1 ? bar0 : mapa_shared(bar0, lead), other0 = CG == 1 ? 0u : mapa_shared(bar0, lead + 1);
       auto commit = [&](uint32_t bar) {   // arrive on this barrier, in both CTAs of a pair, once the MMAs have completed
         if (CG == 1) {
           umma_commit(bar);
         } else {
-          umma_commit_pair(mapa_shared(bar, lead));
-          umma_commit_pair(mapa_shared(bar, lead + 1));
+          umma_commit_pair(own0 + (bar - bar0));
+          umma_commit_pair(other0 + (bar - bar0));
         }
       };
       const uint64_t desc0 = umma_desc_k_sw128(ring);
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
             ok = false;
             break;
           }
-          tc_fence_after();
+          // (no tcgen05 fence: what the barrier announces was written by TMA, not by another thread's tcgen05 operations)
           // descriptor addresses count in 16-byte units; every kind covers 32 bytes of K per instruction
           const uint64_t a_desc = desc0 + (uint64_t)((stage * stage_bytes) >> 4);
           const uint64_t b_desc = a_desc + (kRowsBytes >> 4);
@@ -354,31 +354,26 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       }
     }
   } else if (split == 1) {
-    // ---- epilogue of whole tiles (128 threads) ----
-    const int et = threadIdx.x - 64;
-    const int quad = warp & 3;
+    // ---- epilogue of whole tiles: two warps per 32 rows, which take turns with the 128-byte pieces of the tile's width.
+    // Each works for itself (its 32 rows go through 4 KB of shared memory of its own), so nothing but its own latency
+    // stands between the last MMA and the last store. ----
+    const int quad = warp & 3, turn = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
-    int acc = 0, buf = 0;
+    const uint32_t sb = staging + (uint32_t)(warp - 2) * 4096u;
+    int acc = 0;
     uint32_t acc_phase = 0;
     for (int t = tile0; t < total; t += step) {
-      if (et == 0) {
-        const bool w = mbar_wait(acc_full_bar(acc), acc_phase, p.timeout_ns, abort_flag);
-        if (!w) record_status(p.status, kTimeout, kSiteEpilogue, 0, t, acc);
-        *verdict = w ? 1u : 0u;
-      }
-      named_barrier_sync(1, 128);
-      const bool good = *verdict != 0;
-      named_barrier_sync(1, 128);
-      if (!good) {
-        *abort_flag = 1;
-        break;
-      }
-      tc_fence_after();
       const iris::gemm::TileCoord tc = iris::gemm::raster(t, p.tiles_r, p.tiles_c, p.group);
       const int width = p.glu ? p.tn / 2 : p.tn;   // columns of C in this tile
       const int r0 = (tc.m_idx * CG + pr) * kRows, c0 = tc.n_idx * width;
       const uint32_t src = tmem + lane_addr + acc * kMaxCols;
+      if (!mbar_wait(acc_full_bar(acc), acc_phase, p.timeout_ns, abort_flag)) {
+        if (lane == 0) record_status(p.status, kTimeout, kSiteEpilogue, 0, t, acc);
+        *abort_flag = 1;
+        break;
+      }
+      tc_fence_after();
       auto release = [&]() {
         tc_fence_before();
         __syncwarp();
@@ -390,17 +385,18 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
       if (p.swap) {
         // a thread holds one column of C: the 32 lanes of a store cover neighbouring columns of one row of C
         const int n = r0 + row;
-        for (int c = 0; c < p.tn; c += 16) {
+        for (int c = turn * 16; c < p.tn; c += 32) {
           uint32_t v[16];
           tmem_ld_32x32b_x16(src + c, v);
           tmem_wait_ld();
-          if (c + 16 >= p.tn) release();
           if (n < p.N) st_column<ET>(p.out, (int64_t)(c0 + c) * p.ldo + n, p.ldo, p.M - c0 - c, v);
         }
+        release();
       } else {
         const int pieces = (width + EC - 1) / EC;
+        if (turn >= pieces) release();
 #pragma unroll 1
-        for (int c = 0; c < pieces; ++c) {
+        for (int c = turn; c < pieces; c += 2) {
           uint32_t o[32];   // 128 bytes of this thread's row
           if constexpr (ES == 4) {
             tmem_ld_32x32b_x32(src + c * EC, o);
@@ -440,25 +436,28 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
               }
             }
           }
-          if (c == pieces - 1) release();
-          // two staging buffers: the one written here was read two pieces ago, before the last barrier
-          const uint32_t sb = staging + buf * (kRows * 128);
+          if (c + 2 >= pieces) release();
+          __syncwarp();   // the piece before this one has been read
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            st_shared_v4(sb + row * 128 + ((j ^ (row & 7)) << 4), o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-          named_barrier_sync(1, 128);
+            st_shared_v4(sb + lane * 128 + ((j ^ (lane & 7)) << 4), o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          __syncwarp();
           // out of the buffer with 16-byte stores: 8 lanes cover 128 bytes of a row of C, a warp four rows
           const int left = p.N - (c0 + c * EC), mine = width - c * EC;
           const int bytes = (left < mine ? left : mine) * ES;   // of this piece's row that belong to C
-          uint8_t* base = reinterpret_cast<uint8_t*>(p.out) + ((int64_t)c0 + c * EC) * ES;
+          const int j = lane & 7;
+          if (j * 16 < bytes) {
+            const int64_t pitch = p.ldo * ES;
+            int r = lane >> 3;
+            uint8_t* to = reinterpret_cast<uint8_t*>(p.out) + ((int64_t)c0 + c * EC) * ES + j * 16 +
+                          (r0 + quad * 32 + r) * pitch;
+            const int rows = p.M - (r0 + quad * 32);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int idx = i * 128 + et, r = idx >> 3, j = idx & 7;
-            const uint4 w = ld_shared_v4(sb + r * 128 + ((j ^ (r & 7)) << 4));
-            if (r0 + r < p.M && j * 16 < bytes)
-              *reinterpret_cast<uint4*>(base + (int64_t)(r0 + r) * p.ldo * ES + j * 16) = w;
+            for (int i = 0; i < 8; ++i, r += 4, to += 4 * pitch) {
+              const uint4 w = ld_shared_v4(sb + r * 128 + ((j ^ (r & 7)) << 4));
+              if (r < rows) *reinterpret_cast<uint4*>(to) = w;
+            }
           }
-          buf ^= 1;
         }
       }
       if (++acc == 2) {
@@ -477,6 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
     const int blocks = p.tn / 16;
     const int per = (blocks + split - 1) / split;
     const int quad = warp & 3, row = quad * 32 + lane;
+    const int turn = (warp - 2) >> 2;   // two warps per 32 rows take turns with the blocks
     const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16);
     const iris::gemm::TileCoord tc = iris::gemm::raster(tile0, p.tiles_r, p.tiles_c, p.group);
     const int r = (tc.m_idx * CG + pr) * kRows + row, c0 = tc.n_idx * p.tn;
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
         const int b0 = to * per, b1 = b0 + per < blocks ? b0 + per : blocks;
         const uint32_t peer = mapa_shared(recv, to * CG + pr) + (uint32_t)(slot * per) * kBlock + row * 16;
 #pragma unroll 1
-        for (int b = b0; b < b1 && good; ++b) {
+        for (int b = b0 + turn; b < b1 && good; b += 2) {
           uint32_t v[16];
           tmem_ld_32x32b_x16(acc + b * 16, v);
           tmem_wait_ld();
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
     if (warp >= 2 && good) {
       const int b0 = piece * per, b1 = b0 + per < blocks ? b0 + per : blocks;
 #pragma unroll 1
-      for (int b = b0; b < b1; ++b) {
+      for (int b = b0 + turn; b < b1; b += 2) {
         uint32_t v[16];
         tmem_ld_32x32b_x16(acc + b * 16, v);
         tmem_wait_ld();
@@ -660,34 +660,46 @@ int resident_groups(int c, int sms) {
 }
 
 // Which operand supplies the 128-row tiles, CTA pairs or single CTAs, tile width and pieces of K: the combination with
-// the smallest estimated time.  The estimate (in us) has one term for each thing that was found to bind somewhere; its
-// constants are a fit to 5000 timings of 56 products (1 .. 16384 rows, all four types) in CUDA graphs.  Over those the
-// chosen combination takes 2 % more than the fastest one on average, 28 % at worst (a 4 us product).
-//   * a K block (128 bytes of K) takes the longest of: the MMAs, 2 cycles per column of the tile; 360 cycles of issue;
-//     the loads of the SM at 150 B/ns; the loads of all SMs at 21.7 TB/s out of L2.  Rows that do not start on 128
-//     bytes touch one more L2 line each (17 %);
-//   * reading every operand once at 6.4 TB/s, if that is longer than all K blocks together;
-//   * 3 us per wave of tiles (launch and first loads, or the drain between waves) and 9 ns per column for the epilogue;
-//   * for a split, 0.8 us and 12 ns per column that travels between the CTAs.
+// the smallest estimated time.  The estimate (in us; without what every combination has) has one term for each thing that
+// was found to bind somewhere; its constants are a fit to 14600 timings of 330 products (1 .. 16384 rows, all four types) in
+// CUDA graphs.  Over those the chosen combination takes 2.6 % more than the fastest one on average, 37 % at worst (a 5 us
+// product).
+//   * a K block (128 bytes of K) takes the longest of: the MMAs, 2 cycles per column of the tile; 340 - 400 cycles of issue;
+//     the 1.4 us from one use of a ring slot to the next, shared by the ring's stages; the loads of all SMs at 19 TB/s out
+//     of L2.  Rows that do not start on 128 bytes touch one more L2 line each (12 % and 22 % on the last two), and rows past
+//     the matrix' edge take time although nothing is loaded for them;
+//   * reading every operand once, if that is longer than all K blocks: at 6.8 TB/s, or 8.7 below 50 MB, part of which a
+//     program will find in L2;
+//   * 1.1 us per wave of tiles and 19 ns per column for the epilogue;
+//   * for a split, 1.4 us, and 0.11 us for each piece of 16 columns that a CTA adds up; clusters of three (1 us) and of
+//     five or six (0.1 us) start later than the others.
 double estimate(const Choice& c, int M, int N, int K, int es, int sms) {
   const int kblocks = ceil_div(K * es, 128);
   const int rows = c.swap ? N : M, cols = c.swap ? M : N;
-  const double groups = (double)ceil_div(rows, kRows * c.cg) * ceil_div(cols, c.tn);
-  const int resident = resident_groups(c.cg * c.split, sms);
+  const int tiles_r = ceil_div(rows, kRows * c.cg);
+  const int cluster = c.cg * c.split;
+  const double groups = (double)tiles_r * ceil_div(cols, c.tn);
+  const int resident = resident_groups(cluster, sms);
   const double waves = groups <= resident ? 1.0 : (double)((long long)(groups + resident - 1) / resident);
-  const double ctas = (groups < resident ? groups : resident) * c.cg * c.split;
-  const double load = (kRows + c.tn / c.cg) * 128.0 * ((long long)K * es % 128 ? 1.174 : 1.0);
+  const double ctas = (groups < resident ? groups : resident) * cluster;
+  const bool aligned = (long long)K * es % 128 == 0;
   double per = 2.0 * c.tn / 1900.0;
-  const double issue = (c.cg == 1 ? 358.0 : 365.0) / 1900.0;
+  const double issue = (c.cg == 1 ? 338.0 : 400.0) / 1900.0;
   if (issue > per) per = issue;
-  if (load / 150.1e3 > per) per = load / 150.1e3;
-  if (ctas * load / 21.69e6 > per) per = ctas * load / 21.69e6;
+  const double ring = 1.404 * (aligned ? 1.0 : 1.123) / stages_for(c.cg, c.tn, c.split);
+  if (ring > per) per = ring;
+  const double l2 = ctas * (kRows + c.tn / c.cg) * 128.0 * (aligned ? 1.0 : 1.217) / 18.72e6;
+  if (l2 > per) per = l2;
+  if (!c.swap) per *= 1.0 + 0.49 * (1.0 - (double)rows / ((double)tiles_r * kRows * c.cg));
   double t = waves * ceil_div(kblocks, c.split) * per;
-  const double once = ((double)M * K + (double)N * K + (double)M * N) * es / 6.406e6;
+  const double bytes = ((double)M * K + (double)N * K + (double)M * N) * es;
+  const double once = bytes / (bytes > 50e6 ? 6.8e6 : 8.73e6);
   if (once > t) t = once;
-  t += 3.04 + 0.39 + 0.0087 * c.tn + (waves - 1.0) * 2.94;
-  if (c.split > 1) t += 0.837 + 0.0121 * c.tn * (c.split - 1) / c.split;
-  if (c.swap) t += 0.0011 * c.tn / c.split;
+  t += 0.59 + 0.0188 * c.tn + (waves - 1.0) * 1.1;
+  if (c.split > 1) {
+    t += 1.387 + 0.113 * (c.split - 1) * ceil_div(c.tn / 16, c.split);
+    t += cluster == 3 ? 1.0 : cluster == 5 || cluster == 6 ? 0.1 : 0.0;
+  }
   return t;
 }
 
@@ -698,7 +710,9 @@ void choose(int M, int N, int K, int et, int sms, Choice* best, bool whole = fal
   static const int kSplits[] = {1, 2, 3, 4, 5, 6, 8};
   double best_t = 0;
   best->tn = 0;
-  for (int swap = 0; swap <= (M <= 2 * kRows && !whole ? 1 : 0); ++swap) {
+  // Up to 64 rows the operands always change places: 128-row tiles that lie mostly past the edge load slowly besides
+  // (1 x 22016 x 4096: 44 us against 35).
+  for (int swap = M <= kRows / 2 && !whole ? 1 : 0; swap <= (M <= 2 * kRows && !whole ? 1 : 0); ++swap) {
     const int rows = swap ? N : M, cols = swap ? M : N;
     for (int cg = 1; cg <= (rows > kRows ? 2 : 1); ++cg) {
       for (int tn = grain; tn <= kMaxCols; tn += grain) {
