@@ -629,6 +629,7 @@ struct Choice {
 };
 
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
+int k_blocks(int K, int es) { return (int)(((int64_t)K * es + 127) / 128); }   // blocks of 128 bytes
 
 // Receive buffer of a split tile.  Up to 64 KB it gets room of its own, so that nobody has to wait for the other CTAs'
 // last loads before sending; a larger one would cost too many ring stages and takes the ring's place.
@@ -674,7 +675,7 @@ int resident_groups(int c, int sms) {
 //   * for a split, 1.4 us, and 0.11 us for each piece of 16 columns that a CTA adds up; clusters of three (1 us) and of
 //     five or six (0.1 us) start later than the others.
 double estimate(const Choice& c, int M, int N, int K, int es, int sms) {
-  const int kblocks = ceil_div(K * es, 128);
+  const int kblocks = k_blocks(K, es);
   const int rows = c.swap ? N : M, cols = c.swap ? M : N;
   const int tiles_r = ceil_div(rows, kRows * c.cg);
   const int cluster = c.cg * c.split;
@@ -705,7 +706,7 @@ double estimate(const Choice& c, int M, int N, int K, int es, int sms) {
 
 // `whole`: only forms whose CTAs end with a whole tile (no swap, no split).
 void choose(int M, int N, int K, int et, int sms, Choice* best, bool whole = false) {
-  const int es = elem_size(et), kblocks = ceil_div(K * es, 128);
+  const int es = elem_size(et), kblocks = k_blocks(K, es);
   const int grain = et == kInt8 ? 32 : 16;   // N of an MMA
   static const int kSplits[] = {1, 2, 3, 4, 5, 6, 8};
   double best_t = 0;
@@ -776,7 +777,7 @@ int make_plan(Plan* plan, const void* a, int64_t lda, const void* bt, int64_t ld
     return -1;
   }
   const int es = elem_size(et);
-  if ((N * es) % 16 != 0 || (K * es) % 16 != 0) {
+  if ((int64_t)N * es % 16 != 0 || (int64_t)K * es % 16 != 0) {
     snprintf(g_err, sizeof(g_err), "rows of N and of K elements must be multiples of 16 bytes");
     return -1;
   }
@@ -796,7 +797,7 @@ int make_plan(Plan* plan, const void* a, int64_t lda, const void* bt, int64_t ld
   if (cg > 0) c.cg = cg;
   if (tn > 0) c.tn = tn;
   if (split > 0) c.split = split;
-  const int kblocks = ceil_div(K * es, 128);
+  const int kblocks = k_blocks(K, es);
   if (c.tn < 16 || c.tn > kMaxCols || c.tn % (et == kInt8 ? 32 : 16) != 0 || c.split < 1 ||
       c.split * c.cg > kMaxCluster || c.split > kblocks || c.cg > 2) {
     snprintf(g_err, sizeof(g_err), "tile width %d (a multiple of 16, of 32 for int8, up to 256) or split %d (clusters of "
