@@ -17,17 +17,19 @@
 // out even, heads in groups whose K and V stay in L2.  Roles (320 threads):
 //   warps 0-3, 4-7  softmax of side A, B, one thread per query row: tcgen05.ld of the row of scores, maximum, exp2, row
 //                   sum, and P as 16-bit values back into tensor memory over the scores, where the MMA reads it as its A
-//                   operand.  O stays in tensor memory for all key tiles.  It is rescaled only when the running maximum
-//                   has grown by more than 2^8 since the scale in use was taken (rare after the first tiles; P is then at
-//                   most 256, which changes neither its relative rounding nor that of the fp32 sums).
+//                   operand.  O stays in tensor memory for all key tiles and is rescaled there whenever the running maximum
+//                   of one of the warp's rows has grown, which in most tiles it has.
 //   warp 8          TMA producer: Q tiles, and K / V tiles through a ring of five slots (no multicast)
 //   warp 9          one elected thread issues tcgen05.mma:  S = Q K^T, then O += P V (P from tensor memory, V as an
 //                   MN-major operand: V[key][d] is read as stored), alternating between the sides; the first half of a
 //                   product starts when the first half of P is there
-// What bounds it: the pair form the GPU's power limit (1.17 PFLOP/s without a mask from a rest, less in a long run), the split
-// form the chain scores -> softmax -> product of one side, about 3000 cycles per tile.
+// What bounds it: the chain of one side, scores -> softmax -> product, about 4500 cycles per step of a pair for 2048 of MMAs
+// and 2048 of ex2 (8 x 2048 tokens x 32 heads from a rest: 317 us causal, 514 without a mask), and in a long run the GPU's
+// power limit (302 - 327 and 575 us back to back).  A scale that is renewed only after a growth of 2^8 takes 287 / 467 us
+// instead, but then a row's largest weight is rounded like the others and the error against 64 bits grows by 2 to 4 %
+// (2.034e-3 -> 2.071e-3, 2.256e-3 -> 2.337e-3, both bf16).
 // Before: one 128-row tile per CTA, two threads per row reading the scores twice, P through shared memory, O folded
-// through registers after every tile.  8 x 2048 tokens x 32 heads, causal, bf16: 668 -> 333 us back to back (power-limited), 649 -> 280 us from a rest.
+// through registers after every tile: 659 us causal, 1091 without a mask.
 //
 // Every wait is bounded by timeout_ns: on expiry the CTA records a status, every role leaves its loop, tensor memory
 // is released and the kernel returns.
@@ -61,10 +63,6 @@ constexpr int kBarBytes = 1024;        // barriers and small shared words
 // shared memory: barriers | Q of side A | Q of side B (split: row maxima and sums) | ring
 constexpr int kSmemBytes = 1024 + kBarBytes + (2 + kSlots) * kTileBytes;
 static_assert(kSmemBytes <= 227 * 1024, "shared-memory budget");
-
-// A row's scale is renewed when its maximum has grown by more than this (log2): P is at most 2^8, far from the fp16
-// limit of 65504.
-constexpr float kRescaleStep = 8.f;
 
 // The split form, in which the softmax of a tile is part of the chain that sets the time, makes one in so many pairs of
 // exponentials on the FMA units instead of the special-function unit (1 x 4096 x 4 heads causal: 37.3 -> 33.4 us; every
@@ -498,21 +496,29 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
         const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
         if (j == 0) {
           m_run = mx;
-        } else if (__any_sync(0xffffffffu, mx > m_run + kRescaleStep)) {
-          // rare: take the new maximum and rescale what has been summed.  These scores are complete, so the products
-          // issued before them are too, and the next one waits for P.
-          const float m_new = mx > m_run + kRescaleStep ? mx : m_run;
+        } else if (__any_sync(0xffffffffu, mx > m_run)) {
+          // Each row takes its new maximum at once, so that its largest weight is exactly 1 in the 16 bits of P, and what has
+          // been summed is rescaled.  These scores are complete, so the products issued before them are too, and the next
+          // one waits for P.  (32 columns at a time and two to an instruction: 317 us for 8 x 2048 x 32 causal from a rest;
+          // 16 at a time 328, one to an instruction 322, between the exponentials 336, two loads in flight 328.)
+          const float m_new = fmaxf(m_run, mx);
           const float alpha = m_new == m_run ? 1.f : fast_exp2(m_run - m_new);
+          const float2 alpha2 = make_float2(alpha, alpha);
           l_run *= alpha;
           m_run = m_new;
+          const uint32_t o_x = o_t + x * 128;
 #pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
-            uint32_t o[16];
-            tmem_ld_32x32b_x16(o_t + x * 128 + c * 16, o);
+          for (int c = 0; c < D; c += 32) {
+            uint32_t o[32];
+            tmem_ld_32x32b_x32(o_x + c, o);
             tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32b_x16(o_t + x * 128 + c * 16, o);
+            for (int i = 0; i < 32; i += 2) {
+              const float2 r = mul2(make_float2(__uint_as_float(o[i]), __uint_as_float(o[i + 1])), alpha2);
+              o[i] = __float_as_uint(r.x), o[i + 1] = __float_as_uint(r.y);
+            }
+            tmem_st_32x32b_x16(o_x + c, o);
+            tmem_st_32x32b_x16(o_x + c + 16, o + 16);
           }
         }
         const float2 neg = make_float2(-m_run, -m_run);

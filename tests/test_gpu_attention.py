@@ -71,7 +71,7 @@ def test_attention_large_logits_and_rejects_bad_shapes():
 ])
 def test_attention_both_forms(batch, seq, heads, causal, dtype):
     """The form in which two query tiles share their keys, and the one in which the keys of a query tile are shared out
-    and merged.  Queries grow along the keys' order, so that running maxima move by more than the rescaling step."""
+    and merged.  Queries grow along the keys' order, so that running maxima move from tile to tile."""
     g = torch.Generator(device="cuda").manual_seed(seq + heads)
     t, w = batch * seq, heads * 128
     qkv = torch.randn((t, 3 * w), generator=g, device="cuda")
@@ -121,3 +121,28 @@ def test_attention_keeps_nan_and_infinity_of_a_key(batch, heads, key):
         ref = _reference(bad[:seq], 1, seq, heads, True)[:, :128]
         # as in test_attention_both_forms
         assert (out[:seq, :128].float() - ref).abs().max().item() <= 1.05 * 2.0 ** -7 * bad[:, 2 * w:].float().abs().max().item()
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 1), (2, 40)])   # keys of a query tile shared out; pairs of query tiles
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("key", [260, 390])                  # either side of the split form, not its first tile
+def test_attention_largest_weight_is_exact(batch, heads, key, dtype):
+    """The largest weight of a row is 1 in the 16 bits of P wherever its key lies: one key that weighs 2^x times the others,
+    x from 0.1 to 7, with the only non-zero value, 1.  The output is 1 / (row sum) then, and off by its own rounding alone
+    (half a unit, and 2^-20 for the fp32 sum and the exponentials)."""
+    seq, w = 512, heads * 128
+    qkv = torch.zeros((batch * seq, 3 * w), device="cuda")
+    head = slice(128 * (heads - 1), 128 * heads)              # the last head, the last batch
+    rows = slice((batch - 1) * seq, batch * seq)
+    q, k, v = qkv[rows, :w][:, head], qkv[rows, w:2 * w][:, head], qkv[rows, 2 * w:][:, head]
+    q[:, 3] = torch.linspace(0.8, 55.0, seq, device="cuda")
+    k[key, 3], v[key] = 1.0, 1.0
+    qkv = qkv.to(dtype)
+    out = torch.empty((batch * seq, w), dtype=dtype, device="cuda")
+    attention_fwd(qkv, out, batch, seq, heads, causal=False)
+    x = qkv[rows, :w][:, head][:, 3].double() / 128 ** 0.5    # score of the key, natural logarithm
+    exact = 1.0 / (1.0 + (seq - 1) * torch.exp(-x))
+    bits = 8 if dtype == torch.bfloat16 else 11
+    half = 0.5 * 2.0 ** (torch.floor(torch.log2(exact)) - (bits - 1))
+    err = (out[rows, head].double() - exact[:, None]).abs().amax(1)
+    assert bool((err <= half + exact * 2.0 ** -20).all()), f"up to {(err / half).max().item()} half units"
