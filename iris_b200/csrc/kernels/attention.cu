@@ -109,10 +109,12 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
 }
 // 2^t on the FMA units, for a share of the exponentials (see kPolyEvery).  t = k + f with k the nearest integer, 2^f from a
 // polynomial of degree 5 with value 1 at 0, fitted here for the smallest largest relative error on [-1/2, 1/2]: 9.1e-08 in
-// exact arithmetic, 1.7e-7 evaluated in fp32 (ex2.approx: 2.4e-7).  t below -126 gives 2^-126 instead of 0, a NaN stays one.
+// exact arithmetic, 1.7e-7 evaluated in fp32 (ex2.approx: 2.4e-7).  t below -126.5 gives 0, as ex2.approx.ftz does below -126,
+// so that a masked key weighs nothing however large its value is: k is at least -127, whose scale has the bits of 0.  A NaN
+// stays one.
 __device__ __forceinline__ float2 poly_exp2(float2 t) {
-  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(t.x));   // -126
-  asm("max.NaN.f32 %0, %0, 0fC2FC0000;" : "+f"(t.y));
+  asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(t.x));   // -127
+  asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(t.y));
   const float kMagic = 12582912.f;   // 1.5 * 2^23: the sum's last bits are the integer part
   const float2 r = add2(t, make_float2(kMagic, kMagic));
   const float2 k = add2(r, make_float2(-kMagic, -kMagic));

@@ -146,3 +146,21 @@ def test_attention_largest_weight_is_exact(batch, heads, key, dtype):
     half = 0.5 * 2.0 ** (torch.floor(torch.log2(exact)) - (bits - 1))
     err = (out[rows, head].double() - exact[:, None]).abs().amax(1)
     assert bool((err <= half + exact * 2.0 ** -20).all()), f"up to {(err / half).max().item()} half units"
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 1), (2, 40)])   # keys of a query tile shared out; pairs of query tiles
+def test_attention_masked_keys_weigh_nothing(batch, heads):
+    """The values of later keys reach no query, not even as the smallest normal number times the largest bf16 value: the
+    rows before them have the same bits as with zeros there."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    seq, w = 256, heads * 128
+    qkv = torch.randn((batch * seq, 3 * w), generator=g, device="cuda").to(torch.bfloat16)
+    outs = []
+    for value in (0.0, 3.3e38):
+        late = qkv.clone().view(batch, seq, 3 * w)
+        late[:, 160:, 2 * w:] = value
+        out = torch.empty((batch * seq, w), dtype=torch.bfloat16, device="cuda")
+        attention_fwd(late.view(batch * seq, 3 * w), out, batch, seq, heads, causal=True)
+        outs.append(out.view(batch, seq, w)[:, :160])
+    assert bool(torch.isfinite(outs[0].float()).all())
+    assert torch.equal(outs[0], outs[1])
