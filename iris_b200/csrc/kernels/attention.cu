@@ -523,7 +523,9 @@ __global__ void __launch_bounds__(kThreads, 1) attention_fwd_kernel(const __grid
             tmem_st_32x32b_x16(o_x + c + 16, o + 16);
           }
         }
-        const float2 neg = make_float2(-m_run, -m_run);
+        // (a row that has seen scores of minus infinity only: they weigh 0, and not the NaN of their difference)
+        const float shift = m_run == -INFINITY ? 0.f : -m_run;
+        const float2 neg = make_float2(shift, shift);
         float2 s2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {

@@ -164,3 +164,21 @@ def test_attention_masked_keys_weigh_nothing(batch, heads):
         outs.append(out.view(batch, seq, w)[:, :160])
     assert bool(torch.isfinite(outs[0].float()).all())
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("batch,heads", [(1, 1), (2, 60)])   # keys of a query tile shared out; pairs of query tiles
+@pytest.mark.parametrize("tile", [0, 1, 2])
+def test_attention_tile_of_minus_infinity(batch, heads, tile):
+    """128 keys, a whole tile, whose scores are minus infinity: they weigh nothing, also where they are the first that a
+    row (or its half of the keys) meets."""
+    g = torch.Generator(device="cuda").manual_seed(tile)
+    seq, w = 384, heads * 128
+    qkv = torch.randn((batch * seq, 3 * w), generator=g, device="cuda").to(torch.bfloat16)
+    qkv[:, :128] = qkv[:, :128].abs() + 0.1                   # head 0: positive queries
+    qkv[tile * 128:tile * 128 + 128, w:w + 128] = float("-inf")
+    out = torch.empty((batch * seq, w), dtype=torch.bfloat16, device="cuda")
+    attention_fwd(qkv, out, batch, seq, heads, causal=False)
+    ref = _reference(qkv[:seq], 1, seq, heads, False)
+    # as in test_attention_both_forms
+    bound = 1.05 * 2.0 ** -7 * qkv[:, 2 * w:].float().abs().max().item()
+    assert (out[:seq].float() - ref).abs().max().item() <= bound
