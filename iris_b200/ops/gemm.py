@@ -209,13 +209,18 @@ class FusedGemm:
         self.a, self.bt = a_use, bt
         dev = c0.device
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        self.swiglu = bool(swiglu)
         # One rank: nothing to exchange, so the product goes straight into the output (csrc/kernels/gemm_local.cu), unless
-        # the caller asks for a schedule of the fused kernel or for its trace.
-        self.local = (self.world == 1 and not trace and not nvls and "IRIS_STREAM_K" not in os.environ and all(
+        # the caller asks for a schedule of the fused kernel or for its trace, or the output is not just the product: a
+        # buffer of another width (the fused kernel stores through a tensor map and so keeps to `c_cols` columns), or a
+        # larger one whose rest the adding form clears.
+        whole = self.swiglu or mode in ("one_shot", "two_shot") or not c_cols or int(c_cols) == self.N
+        if mode == "reduce" and out is not None and tuple(out[0].shape) != (self.M, self.N):
+            whole = False
+        self.local = (self.world == 1 and whole and not trace and not nvls and "IRIS_STREAM_K" not in os.environ and all(
             x is None for x in (ctas_per_rank, group_m, cta_group, stream_k, push, ksplit, bn, tail_split, push_kind)))
         if self.local:
             stream_k = False
-        self.swiglu = bool(swiglu)
         if self.swiglu:
             if not (self.local and mode == "store" and self.N % 2 == 0 and self.dtype in (torch.bfloat16, torch.float16)):
                 raise ValueError("swiglu=True: one rank, mode 'store', 16-bit elements, an even number of rows of B and no "

@@ -270,3 +270,59 @@ def test_stream_k_default_rule(monkeypatch):
     monkeypatch.setenv("IRIS_STREAM_K", "1")
     assert plan_gemm(1024, 8192, 8192, **one).sk_units > 0
     assert plan_gemm(8192, 3584, 4096, stream_k=False, **one).sk_units == 0   # an explicit argument wins
+
+
+class FakeLocalKernels(FakeKernels):
+    """The one-rank entry points as well: records what a plan is created from."""
+
+    def __init__(self):
+        super().__init__()
+        self.local = []
+
+    def iris_gemm_local_create(self, *args):
+        self.local.append(dict(zip(("a", "lda", "bt", "ldb", "out", "ldo", "M", "N", "K"), args[:9]), glu=args[-1]))
+        return 1000 + len(self.local)
+
+    def iris_gemm_local_info(self, h, info):
+        pass
+
+    def iris_gemm_local_destroy(self, h):
+        pass
+
+
+@pytest.fixture()
+def world1(monkeypatch):
+    ctx = iris.Iris.local_world(1, heap_size=64 << 20, backend="cpu")[0]
+    fake = FakeLocalKernels()
+    monkeypatch.setattr(G, "_lib", lambda: fake)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: SimpleNamespace(multi_processor_count=148))
+    monkeypatch.delenv("IRIS_STREAM_K", raising=False)
+    ctx.backend = "cuda"
+    yield ctx, fake
+    ctx.backend = "cpu"
+    ctx.close()
+
+
+def test_one_rank_kernel_only_where_the_output_is_the_product(world1):
+    """A width of the output (``c_cols``) other than the product's is kept to by the fused kernel's tensor map, which cuts
+    the product off there; the one-rank kernel writes whole rows of the product."""
+    ctx, fake = world1
+    (a,), (bt,) = _ab(256, 512, 128, 1)
+    for c_cols, rows in ((320, 256), (640, 256)):
+        op = G.FusedGemm(ctx, [a], [bt], "store", c_cols=c_cols)
+        assert not op.local and not fake.local
+        assert (fake.descs[-1].c_cols, fake.descs[-1].ldc, fake.descs[-1].N) == (c_cols, c_cols, 512)
+        assert op.out[0].shape == (rows, c_cols)
+    # the adding form clears all of the output, also what lies beside the product
+    wide = ctx.zeros((256, 640), dtype=torch.bfloat16)
+    assert not G.FusedGemm(ctx, [a], [bt], "reduce", store_all=True, out=[wide]).local
+    for kw in (dict(mode="store"), dict(mode="store", c_cols=512), dict(mode="reduce", store_all=True),
+               dict(mode="reduce", store_all=True, out=[wide[:, :512]]), dict(mode="one_shot"),
+               dict(mode="store", out=[wide[:, 64:576]])):
+        op = G.FusedGemm(ctx, [a], [bt], **kw)
+        assert op.local, kw
+        got = fake.local[-1]
+        assert (got["M"], got["N"], got["K"], got["glu"]) == (256, 512, 128, 0)
+        assert got["out"] == op.out[0].data_ptr() and got["ldo"] == op.out[0].stride(0) >= 512
+    op = G.FusedGemm(ctx, [a], [bt], "store", swiglu=True)
+    assert op.local and (fake.local[-1]["N"], fake.local[-1]["ldo"], fake.local[-1]["glu"]) == (256, 256, 1)

@@ -139,6 +139,34 @@ def test_choice_matches_and_repeats(m, n, k, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["store", "reduce"])
+@pytest.mark.parametrize("c_cols", [320, 328])
+def test_narrower_output_cuts_the_product_off(mode, c_cols):
+    """``c_cols`` below the rows of B: the columns from there on are not written, not to the next row and not past the
+    buffer's end (a guard band of 3s all round)."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import iris_b200 as iris
+    from iris_b200.ops import gemm as G
+    m, n, k = 256, 512, 192
+    a, bt = _operand((m, k), "bf16", 1), _operand((n, k), "bf16", 2)
+    ctx = iris.iris(64 << 20)
+    frame = ctx.full((m + 2, 336), 3, dtype=torch.bfloat16)
+    op = G.FusedGemm(ctx, [a], [bt], mode, store_all=mode == "reduce", out=[frame[1:m + 1, :c_cols]], c_cols=c_cols)
+    got = op()[0]
+    op.check()
+    _check(got, a, bt[:c_cols])
+    frame[1:m + 1, :c_cols] = 3
+    assert bool((frame == 3).all()), "wrote outside the output"
+    own = G.FusedGemm(ctx, [a], [bt], mode, store_all=mode == "reduce", c_cols=320)
+    own()
+    own.check()
+    assert own.out[0].shape == (m, 320)
+    _check(own.out[0], a, bt[:320])
+    op.close(), own.close(), ctx.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,inter,k,dtype", [(1, 8, 64, "bf16"), (128, 1376, 512, "bf16"), (129, 200, 264, "fp16"),
                                              (700, 2744, 1032, "bf16"), (2048, 1024, 512, "fp16")])
 def test_gate_and_linear_projection_in_one(m, inter, k, dtype):
