@@ -786,6 +786,10 @@ int make_plan(Plan* plan, const void* a, int64_t lda, const void* bt, int64_t ld
     snprintf(g_err, sizeof(g_err), "base addresses and row pitches must be multiples of 16 bytes");
     return -1;
   }
+  if (M > 1 && ldo < N) {   // (the operands' rows may overlap: they are only read)
+    snprintf(g_err, sizeof(g_err), "the output's row pitch is smaller than its rows");
+    return -1;
+  }
   const int sms = prepare_device(device);
   if (sms < 1) {
     snprintf(g_err, sizeof(g_err), "device %d cannot be set up for the kernel", device);

@@ -103,6 +103,11 @@ def _check_operand(t: torch.Tensor, name: str, dtype: Optional[torch.dtype] = No
         raise ValueError(f"{name}: base address and row pitch must be multiples of 16 bytes")
 
 
+def _reachable(t: torch.Tensor, device: torch.device) -> bool:
+    """Whether kernels on ``device`` may touch ``t``: its own memory, or page-locked host memory."""
+    return t.device == device or (t.device.type == "cpu" and t.is_pinned())
+
+
 def as_kmajor_bt(b: torch.Tensor) -> torch.Tensor:
     """Accept ``B`` as ``[K, N]`` with strides ``(1, ld)`` (the reference's ``randn(n, k).T``) or as ``Bt = [N, K]``
     with a contiguous last dimension, and return the ``[N, K]`` K-major view."""
@@ -266,6 +271,12 @@ class FusedGemm:
             c_rows, part_row0, out_row0 = 0, (0, 0), -1
         for o in self.out:
             _check_operand(o, "output", self.dtype)
+            if o.shape[0] < pl.out_rows or o.shape[1] < c_cols_eff:
+                raise ValueError(f"output: [{pl.out_rows}, {c_cols_eff}] or larger, got {tuple(o.shape)}")
+        if self.local:
+            for t, name in ((a_use[0], "A"), (bt[0], "B"), (self.out[0], "output")):
+                if not _reachable(t, dev):
+                    raise ValueError(f"{name} is on {t.device}, the context on {dev}")
         d = _Desc()
         for l, ctx in enumerate(self.ctxs):
             d.a_ptr[l], d.lda[l] = a_use[l].data_ptr(), a_use[l].stride(0)
@@ -353,7 +364,7 @@ class FusedGemm:
             if not self._plan:
                 raise RuntimeError("fused GEMM plan: " + lib.iris_gemm_last_error().decode())
             self.ctas_per_rank = lib.iris_gemm_plan_ctas_per_rank(self._plan)  # what fits on the device
-        if self.local:   # the fused plan has vetted the arguments; what runs is the one-rank kernel
+        if self.local:   # the fused plan has vetted sizes and schedule (swiglu: checked above); the one-rank kernel runs
             if not self.swiglu:
                 lib.iris_gemm_plan_destroy(self._plan)
             a0, b0, o0 = a_use[0], bt[0], self.out[0]
@@ -569,16 +580,19 @@ def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
         _private_ctx[dev] = ctx
     bt = as_kmajor_bt(bt)
     n = bt.shape[0]
+    device = a.get_device()
     if out is None:
         out = a.new_empty((a.shape[0], n))
-    if cta_group is None and bn is None and tail_split is None and "IRIS_STREAM_K" not in os.environ:
+    if (cta_group is None and bn is None and tail_split is None and "IRIS_STREAM_K" not in os.environ
+            and bt.get_device() == device and out.get_device() == device):
         _check_operand(bt, "B")
         _check_operand(a, "A", bt.dtype)
         m, k = a.shape
         if k != bt.shape[1]:
             raise ValueError(f"K mismatch: A has {k}, B has {bt.shape[1]}")
         _check_operand(out, "output", bt.dtype)
-        device = a.get_device()
+        if out.shape[0] < m or out.shape[1] < n:
+            raise ValueError(f"output: [{m}, {n}] or larger, got {tuple(out.shape)}")
         raw = _native.current_stream(device)
         lib = _lib()
         rc = lib.iris_gemm_local(a.data_ptr(), a.stride(0), bt.data_ptr(), bt.stride(0), out.data_ptr(), out.stride(0), m, n, k,
@@ -590,11 +604,13 @@ def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
             t.record_stream(stream)
         return out
     mark = ctx.mark()
-    op = FusedGemm(ctx, [a], [bt], "store", out=[out], cta_group=cta_group, bn=bn, tail_split=tail_split)
-    op()
-    op.close()
-    torch.cuda.current_stream(dev).synchronize()  # the plan's flags and workspace are released just below
-    ctx.reset(mark)
+    try:
+        op = FusedGemm(ctx, [a], [bt], "store", out=[out], cta_group=cta_group, bn=bn, tail_split=tail_split)
+        op()
+        op.close()
+        torch.cuda.current_stream(dev).synchronize()  # the plan's flags and workspace are released just below
+    finally:
+        ctx.reset(mark)
     return out
 
 

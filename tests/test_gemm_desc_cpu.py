@@ -326,3 +326,65 @@ def test_one_rank_kernel_only_where_the_output_is_the_product(world1):
         assert got["out"] == op.out[0].data_ptr() and got["ldo"] == op.out[0].stride(0) >= 512
     op = G.FusedGemm(ctx, [a], [bt], "store", swiglu=True)
     assert op.local and (fake.local[-1]["N"], fake.local[-1]["ldo"], fake.local[-1]["glu"]) == (256, 256, 1)
+
+
+def test_outputs_and_devices_are_checked_before_any_launch(world1, monkeypatch):
+    ctx, fake = world1
+    (a,), (bt,) = _ab(256, 512, 128, 1)
+    z = lambda *s: torch.zeros(s, dtype=torch.bfloat16)
+    for kw in (dict(out=[z(255, 512)]), dict(out=[z(256, 504)]), dict(out=[z(256, 512)[:, :256]]),
+               dict(out=[z(256, 248)], swiglu=True), dict(out=[z(255, 256)], swiglu=True),
+               dict(out=[z(256, 320)], c_cols=512), dict(out=[z(128, 512)], bn=64)):
+        with pytest.raises(ValueError, match="output"):
+            G.FusedGemm(ctx, [a], [bt], "store", **kw)
+    assert not fake.local and not fake.descs
+    G.FusedGemm(ctx, [a], [bt], "store", out=[z(300, 520)])          # a larger buffer is as good
+    G.FusedGemm(ctx, [a], [bt], "store", out=[z(256, 256)], swiglu=True)
+    assert len(fake.local) == 2
+    monkeypatch.setattr(ctx, "device", torch.device("cuda", 0))      # operands in ordinary host memory
+    for kw in (dict(), dict(swiglu=True)):
+        with pytest.raises(ValueError, match="A is on cpu, the context on cuda:0"):
+            G.FusedGemm(ctx, [a], [bt], "store", out=[z(256, 512)], **kw)
+    assert len(fake.local) == 2
+
+
+def test_gemm_checks_its_output_before_the_launch(monkeypatch):
+    """``gemm`` on stand-ins that claim to be on a GPU: an output too small, or operands elsewhere, reach no kernel."""
+    calls = []
+
+    class Kernels(FakeLocalKernels):
+        def iris_gemm_local(self, *args):
+            calls.append(args)
+            return 0
+
+    class OnGpu(torch.Tensor):
+        def get_device(self):
+            return 0
+
+        def record_stream(self, stream):
+            pass
+
+    ctx = iris.Iris.local_world(1, heap_size=64 << 20, backend="cpu")[0]
+    ctx.backend = "cuda"
+    monkeypatch.setattr(G, "_lib", lambda fake=Kernels(): fake)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda dev: SimpleNamespace(multi_processor_count=148))
+    monkeypatch.setitem(G._private_ctx, torch.device("cpu"), ctx)
+    monkeypatch.setattr(G._native, "current_stream", lambda device: 0)
+    monkeypatch.setattr(G, "_stream_object", lambda device, raw: None)
+    monkeypatch.delenv("IRIS_STREAM_K", raising=False)
+    gpu = lambda *s: torch.zeros(s, dtype=torch.bfloat16).as_subclass(OnGpu)
+    a, bt = gpu(256, 128), gpu(512, 128)
+    for out in (gpu(255, 512), gpu(256, 504), gpu(256, 512)[:, :256]):
+        with pytest.raises(ValueError, match="output"):
+            G.gemm(a, bt, out=out)
+    assert not calls
+    for out in (gpu(256, 512), gpu(300, 520)[:, :512], gpu(300, 520), None):
+        G.gemm(a, bt, out=out)
+    assert len(calls) == 4 and all((c[6], c[7], c[8]) == (256, 512, 128) for c in calls)
+    # not all on the GPU of `a`: left to the prepared op, which looks at each
+    monkeypatch.setattr(ctx, "device", torch.device("cuda", 0))
+    with pytest.raises(ValueError, match="is on cpu"):
+        G.gemm(a, torch.zeros((512, 128), dtype=torch.bfloat16))
+    assert len(calls) == 4
+    ctx.backend, ctx.device = "cpu", torch.device("cpu")
+    ctx.close()

@@ -42,6 +42,17 @@ def test_choice_is_launchable_for_every_size():
         assert not (swap and m > 256)
 
 
+@pytest.mark.skipif(not _native.kernels_available(), reason="native kernels not built")
+def test_overlapping_output_rows_are_refused():
+    """Before any device is looked at; a single row has no pitch."""
+    from iris_b200.ops import gemm as G
+    lib = G._lib()
+    for m, glu, refused in ((2, 0, True), (2, 1, True), (1, 0, False)):
+        h = lib.iris_gemm_local_create(4096, 64, 8192, 64, 12288, 248, m, 256, 64, 0, -1, 0, 0, -1, 0, 0, 0, glu)
+        assert h is None
+        assert (b"row pitch is smaller" in lib.iris_gemm_local_last_error()) == refused
+
+
 def _operand(shape, dtype, seed):
     g = torch.Generator(device="cuda").manual_seed(seed)
     if dtype == "int8":
