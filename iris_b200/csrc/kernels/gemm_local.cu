@@ -514,10 +514,11 @@ __global__ void __launch_bounds__(kThreads, 1) local_gemm_kernel(const __grid_co
             st_cluster_v4(at + j * (kRows * 16), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
       }
-      // one fence for all of it, then relaxed arrivals (a release per owner would wait for the stores each time);
-      // after a failure they are made too, so that no one waits for this CTA
-      fence_acq_rel_cluster();
+      // One fence for all of it, then relaxed arrivals (a release per owner would wait for the stores each time).  The
+      // fence comes after the warp's barrier: an arriving lane releases what it knows by its fence, and by the barrier it
+      // knows the stores of all lanes.  After a failure the arrivals are made too, so that no one waits for this CTA.
       __syncwarp();
+      fence_acq_rel_cluster();
       if (lane < split && lane != piece && lane * per < blocks)
         mbar_arrive_cluster_relaxed(mapa_shared(recv_bar, lane * CG + pr));
     }

@@ -330,7 +330,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// The same without ordering of its own: after a fence_acq_rel_cluster() of the threads whose writes it announces.
+// The same without ordering of its own.  The arriving thread itself must have made a fence_acq_rel_cluster() before, after
+// it had synchronised with the threads whose writes it announces (__syncwarp(), a block barrier): what it knew then is
+// what the arrival releases.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

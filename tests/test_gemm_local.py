@@ -6,7 +6,9 @@ Bounds: the operands are multiplied exactly and summed in fp32 (int8: in 32-bit 
 its rounding, half a unit in the last of 8 (bf16) or 11 (fp16) bits, at most 2^-8 or 2^-11 of the value, plus the fp32 sums' K * 2^-24 of the sum of magnitudes; a tf32
 product rounds each operand to 11 bits, so every term is off by at most 2 * 2^-11 of its magnitude.  int8 is exact."""
 import ctypes
+import os
 import random
+import re
 
 import pytest
 import torch
@@ -51,6 +53,31 @@ def test_overlapping_output_rows_are_refused():
         h = lib.iris_gemm_local_create(4096, 64, 8192, 64, 12288, 248, m, 256, 64, 0, -1, 0, 0, -1, 0, 0, 0, glu)
         assert h is None
         assert (b"row pitch is smaller" in lib.iris_gemm_local_last_error()) == refused
+
+
+def test_split_handover_publishes_the_stores_of_every_lane():
+    """The order in which a warp hands its partial sums over, read out of the source and run through the memory model's
+    happens-before relation: each of 32 lanes stores into another CTA's shared memory, and what a relaxed arrival
+    publishes is what its own thread knew at its last fence.  A thread knows its own stores and, after a warp barrier,
+    those of all lanes; the arrivals have to publish all 32."""
+    source = open(os.path.join(os.path.dirname(_native.__file__), "csrc", "kernels", "gemm_local.cu")).read()
+    part = source[source.index("st_cluster_v4(at"):source.index("cluster_arrive();   // nothing more is sent")]
+    part = re.sub(r"//[^\n]*", "", part)
+    order = re.findall(r"\b(st_cluster_v4|__syncwarp|fence_acq_rel_cluster|mbar_arrive_cluster_relaxed)\(", part)
+    order = order[:order.index("mbar_arrive_cluster_relaxed") + 1]
+    assert order[0] == "st_cluster_v4"
+    knows = [set() for _ in range(32)]
+    released = [set() for _ in range(32)]
+    for what in order:
+        if what == "st_cluster_v4":
+            for lane in range(32):
+                knows[lane].add(lane)
+        elif what == "__syncwarp":
+            everything = set().union(*knows)
+            knows = [set(everything) for _ in range(32)]
+        elif what == "fence_acq_rel_cluster":
+            released = [set(k) for k in knows]
+    assert all(r == set(range(32)) for r in released)
 
 
 def _operand(shape, dtype, seed):
