@@ -15,7 +15,9 @@ namespace {
 
 // All kernels here are launched with programmatic stream serialization and begin with this: their blocks are placed while
 // the kernel in front drains, and the blocks of the next kernel (a GEMM or attention with a set-up of microseconds) while
-// these finish.  Nothing is read or written before the wait.
+// these finish.  Nothing is read or written before the wait, and no pointer is __restrict__: the kernel in front may write
+// what these read while their blocks exist, so no load may be taken for one of constant data (read through the
+// non-coherent path, or lifted over the wait).
 // (Decoder of four layers, 256 tokens: 561 -> 555 us.)
 __device__ __forceinline__ void begin() {
   iris::ptx::grid_dependency_wait();
@@ -41,9 +43,9 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 
 // One CTA per row; cols % 8 == 0.  out[r, :] = x[r, :] * rsqrt(mean(x^2) + eps) * w
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
-                                                           const __nv_bfloat16* __restrict__ w,
-                                                           __nv_bfloat16* __restrict__ out, int64_t ldo, int cols,
+__global__ void __launch_bounds__(kThreads) rmsnorm_kernel(const __nv_bfloat16* x, int64_t ldx,
+                                                           const __nv_bfloat16* w,
+                                                           __nv_bfloat16* out, int64_t ldo, int cols,
                                                            float eps) {
   __shared__ float red[kThreads / 32];
   begin();
@@ -80,9 +82,9 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_kernel(const __nv_bfloat16* 
 // As above for rows of at most kThreads * VPT vectors: the row stays in registers between the two passes, so x is
 // read once (the generic kernel's second read hits L2 but costs a second round of load latency per row).
 template <int kThreads, int VPT>
-__global__ void __launch_bounds__(kThreads) rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
-                                                               const __nv_bfloat16* __restrict__ w,
-                                                               __nv_bfloat16* __restrict__ out, int64_t ldo, int cols,
+__global__ void __launch_bounds__(kThreads) rmsnorm_reg_kernel(const __nv_bfloat16* x, int64_t ldx,
+                                                               const __nv_bfloat16* w,
+                                                               __nv_bfloat16* out, int64_t ldo, int cols,
                                                                float eps) {
   __shared__ float red[kThreads / 32];
   begin();
@@ -137,10 +139,10 @@ __global__ void __launch_bounds__(kThreads) rmsnorm_reg_kernel(const __nv_bfloat
 // written once, instead of the three reads and two writes of the two separate kernels.  Rows of at most
 // kThreads * VPT vectors.
 template <int kThreads, int VPT>
-__global__ void __launch_bounds__(kThreads) add_rmsnorm_reg_kernel(__nv_bfloat16* __restrict__ x, int64_t ldx,
-                                                                   const __nv_bfloat16* __restrict__ y, int64_t ldy,
-                                                                   const __nv_bfloat16* __restrict__ w,
-                                                                   __nv_bfloat16* __restrict__ out, int64_t ldo,
+__global__ void __launch_bounds__(kThreads) add_rmsnorm_reg_kernel(__nv_bfloat16* x, int64_t ldx,
+                                                                   const __nv_bfloat16* y, int64_t ldy,
+                                                                   const __nv_bfloat16* w,
+                                                                   __nv_bfloat16* out, int64_t ldo,
                                                                    int cols, float eps) {
   __shared__ float red[kThreads / 32];
   begin();
@@ -208,8 +210,8 @@ __device__ __forceinline__ float silu_mul(float a, float b) {
 // out[r, c] = silu(gu[r, c]) * gu[r, inter + c]; four independent 16-byte load pairs in flight per thread.
 // Index: 32-bit (fewer instructions than 64-bit division) unless the matrix has 2^31 vectors or more.
 template <class Index>
-__global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* __restrict__ gu, int64_t ldg,
-                                                     __nv_bfloat16* __restrict__ out, int64_t ldo, int rows, int inter) {
+__global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* gu, int64_t ldg,
+                                                     __nv_bfloat16* out, int64_t ldo, int rows, int inter) {
   constexpr int U = 4;
   begin();
   const Index nv = (Index)(inter / 8);
@@ -245,7 +247,7 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* __rest
 }
 
 // x[r, :] += y[r, :]
-__global__ void residual_add_kernel(__nv_bfloat16* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ y,
+__global__ void residual_add_kernel(__nv_bfloat16* x, int64_t ldx, const __nv_bfloat16* y,
                                     int64_t ldy, int rows, int cols) {
   begin();
   const int nv = cols / 8;
