@@ -804,6 +804,7 @@ int iris_k_attention_fwd(const void* qkv, int64_t ld_qkv, void* out, int64_t ldo
   void* args[] = {&p};
   e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), args);
   if (e != cudaSuccess) {
+    (void)cudaGetLastError();   // reported here: it must not turn up at someone else's launch
     snprintf(g_attn_err, sizeof(g_attn_err), "attention: launch: %s", cudaGetErrorString(e));
     return -3;
   }

@@ -280,7 +280,9 @@ int launch(void (*kernel)(P...), int grid, int block, void* stream, A... args) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) == cudaSuccess ? 0 : -1;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) == cudaSuccess) return 0;
+  (void)cudaGetLastError();   // reported here: it must not turn up at someone else's launch
+  return -1;
 }
 
 }  // namespace

@@ -758,13 +758,17 @@ int prepare_device(int device) {
   if (device < 0 || device >= kMaxDevices) return 0;
   std::call_once(once[device], [&]() {
     int prev = -1, n = 0;
-    if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return;
+    if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return;
+    }
     bool fine = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
     for (int i = 0; i < 8; ++i)
       fine = fine && cudaFuncSetAttribute(kernel_for(i / 2, 1 + i % 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           kSmemMax) == cudaSuccess;
     cudaSetDevice(prev);
     if (fine) sms[device] = n;
+    else (void)cudaGetLastError();
   });
   return sms[device];
 }
@@ -847,6 +851,7 @@ int make_plan(Plan* plan, const void* a, int64_t lda, const void* bt, int64_t ld
 int launch(const Plan* plan, void* stream) {
   int prev = -1;
   if (cudaGetDevice(&prev) != cudaSuccess || (prev != plan->device && cudaSetDevice(plan->device) != cudaSuccess)) {
+    (void)cudaGetLastError();
     snprintf(g_err, sizeof(g_err), "device %d cannot be made current", plan->device);
     return -1;
   }
@@ -868,6 +873,7 @@ int launch(const Plan* plan, void* stream) {
   const cudaError_t e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel_for(plan->et, plan->cg)), args);
   if (prev != plan->device) cudaSetDevice(prev);
   if (e != cudaSuccess) {
+    (void)cudaGetLastError();   // reported here: it must not turn up at someone else's launch
     snprintf(g_err, sizeof(g_err), "launch failed: %s", cudaGetErrorString(e));
     return -1;
   }
