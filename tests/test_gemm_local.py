@@ -4,7 +4,8 @@ with remainders in every dimension.
 
 Bounds: the operands are multiplied exactly and summed in fp32 (int8: in 32-bit integers), so a 16-bit result is off by
 its rounding, half a unit in the last of 8 (bf16) or 11 (fp16) bits, at most 2^-8 or 2^-11 of the value, plus the fp32 sums' K * 2^-24 of the sum of magnitudes; a tf32
-product rounds each operand to 11 bits, so every term is off by at most 2 * 2^-11 of its magnitude.  int8 is exact."""
+product cuts each operand to 11 bits, so every term is off by at most 2 * 2^-10 of its magnitude, and the sums of 256 terms
+and more here, whose cuts average out, by at most 2 * 2^-11.  int8 is exact."""
 import ctypes
 import os
 import random
@@ -100,7 +101,7 @@ def _check(got, a, bt):
     assert bool(((got.double() - exact).abs() <= 1.01 * bound).all())
 
 
-def _run(a, bt, out, swap=-1, cg=0, tn=0, split=0, stream=None):
+def _run(a, bt, out, swap=-1, cg=0, tn=0, split=0):
     from iris_b200.ops import gemm as G
     lib = G._lib()
     status = torch.zeros(16, dtype=torch.int32, device="cuda")
@@ -130,6 +131,50 @@ def test_every_form_against_float64(dtype, cg, split, swap):
             _check(out, a, bt)
             frame[1:m + 1, g:g + n] = 3
             assert bool((frame == 3).all()), "wrote outside the output"
+
+
+WIDTHS = {"bf16": (48, 112, 176, 256), "fp16": (16, 128, 192, 240), "fp32": (16, 48, 96, 256), "int8": (32, 96, 160, 256)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kblocks", [1, 19])    # a tile's loads: a fraction of the ring, or several times round it
+@pytest.mark.parametrize("dtype", list(TYPES))
+@pytest.mark.parametrize("cg", [1, 2])
+@pytest.mark.parametrize("swap", [0, 1])
+def test_many_tiles_per_cta(dtype, cg, swap, kblocks):
+    """Every form with at least five tiles for every CTA (or pair): two accumulators are in flight, so from the third tile
+    on the MMAs wait for an accumulator that the epilogue gives back.  Tile widths of one to eight 128-byte pieces."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from iris_b200.ops import gemm as G
+    lib, es = G._lib(), SIZE[dtype]
+    g = 16 // es
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    status = torch.zeros(16, dtype=torch.int32, device="cuda")
+    k = kblocks * 128 // es - (g if kblocks > 1 else 0)
+    for i, tn in enumerate(WIDTHS[dtype]):
+        tiles_r = 13
+        tiles_c = -(-11 * (sms // cg) // (2 * tiles_r)) + 1
+        rows, cols = (tiles_r - 1) * 128 * cg + 96, (tiles_c - 1) * tn + 16     # the last tile of either side is not full
+        m, n = (cols, rows) if swap else (rows, cols)
+        a, bt = _operand((m, k), dtype, i), _operand((n, k), dtype, i + 9)
+        if dtype == "fp32":   # 11 significant bits, which tf32 holds: with one K block the cut bits do not average out
+            a, bt = ((x.view(torch.int32) & -8192).view(torch.float32) for x in (a, bt))
+        frame = torch.full((m + 2, n + 2 * g), 3, dtype=TYPES[dtype], device="cuda")
+        out = frame[1:m + 1, g:g + n]
+        h = lib.iris_gemm_local_create(a.data_ptr(), k, bt.data_ptr(), k, out.data_ptr(), out.stride(0), m, n, k, CODE[dtype], 0,
+                                       status.data_ptr(), 2000000000, swap, cg, tn, 1, 0)
+        assert h, lib.iris_gemm_local_last_error().decode()
+        info = (ctypes.c_int * 6)()
+        lib.iris_gemm_local_info(h, info)
+        assert list(info)[:4] == [swap, cg, tn, 1] and tiles_r * tiles_c >= 5 * (info[4] // cg)
+        assert lib.iris_gemm_local_launch(h, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        lib.iris_gemm_local_destroy(h)
+        assert int(status[0]) == 0
+        _check(out, a, bt)
+        frame[1:m + 1, g:g + n] = 3
+        assert bool((frame == 3).all()), "wrote outside the output"
 
 
 @pytest.mark.gpu
@@ -206,7 +251,8 @@ def test_narrower_output_cuts_the_product_off(mode, c_cols):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,inter,k,dtype", [(1, 8, 64, "bf16"), (128, 1376, 512, "bf16"), (129, 200, 264, "fp16"),
-                                             (700, 2744, 1032, "bf16"), (2048, 1024, 512, "fp16")])
+                                             (700, 2744, 1032, "bf16"), (2048, 1024, 512, "fp16"),
+                                             (4096, 8200, 264, "bf16"), (4000, 8192, 1288, "fp16")])
 def test_gate_and_linear_projection_in_one(m, inter, k, dtype):
     """``swiglu=True`` against silu(a gate^T) * (a linear^T) in float64.  Off by the output's rounding, by the fp32 sums'
     K * 2^-24 of their magnitudes (times what either factor scales them by; silu' <= 1.1), and by 2^-20 of the value for
@@ -218,7 +264,7 @@ def test_gate_and_linear_projection_in_one(m, inter, k, dtype):
     a = _operand((m, k), dtype, 1)
     bt = (_operand((2 * inter, k), dtype, 2).float() / k ** 0.5).to(TYPES[dtype])
     frame = torch.full((m, inter + 16), 3, dtype=TYPES[dtype], device="cuda")
-    ctx = iris.iris(128 << 20)
+    ctx = iris.iris(256 << 20)
     op = G.all_gather_gemm(ctx, (m + 127) // 128 * 128, [bt], swiglu=True)
     op.a_full[0][:m].copy_(a)
     got = op()[0][:m]
@@ -226,6 +272,9 @@ def test_gate_and_linear_projection_in_one(m, inter, k, dtype):
     own = G.FusedGemm(ctx, [a], [bt], "store", out=[frame[:, 8:8 + inter]], swiglu=True)
     own()
     own.check()
+    if m >= 4000:   # several tiles for every CTA or pair, see test_many_tiles_per_cta
+        tiles = -(-m // (128 * own.cta_group)) * -(-inter // (own.bn // 2))
+        assert tiles > 2 * (own.ctas_per_rank // own.cta_group)
     assert got.shape == (m, inter) and torch.equal(frame[:, 8:8 + inter], got)
     assert bool((frame[:, :8] == 3).all()) and bool((frame[:, 8 + inter:] == 3).all())
     g, u = a.double() @ bt[:inter].double().t(), a.double() @ bt[inter:].double().t()
