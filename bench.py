@@ -179,11 +179,16 @@ def main() -> int:
         if world > 1 and not args.no_selfcheck:
             selfcheck = run_selfcheck(ctx, G, torch, dist, dev, rank, world, barrier)
 
+        def start_sampler():
+            """Clock samples on rank 0 while an arm runs, device-timed and end to end (both arms with it alike)."""
+            if rank != 0:
+                return None
+            s = ClockSampler(local_rank, period_ms=10).start()
+            s.wait_first_sample(10.0)
+            return s
+
         # ---- device-timed kernel-only measurement ----
-        sampler = None
-        if rank == 0:
-            sampler = ClockSampler(local_rank, period_ms=10).start()
-            sampler.wait_first_sample(10.0)
+        sampler = start_sampler()
         for _ in range(args.warmup):
             op()
         launches0 = op.launches
@@ -275,6 +280,7 @@ def main() -> int:
                 torch.matmul(a_dev, b_kn, out=c_part)
                 if world > 1:
                     dist.all_gather_into_tensor(gathered, c_part)
+            sampler = start_sampler()
             for _ in range(args.warmup):
                 unfused()
             bst = _stats(timed_steps(unfused, args.steps))
@@ -296,8 +302,9 @@ def main() -> int:
                     return gathered[:, 0, :]     # row 0 of C: one piece per rank's column block
                 return c_part[0]
             base_e2e_ms = time_e2e(base_step, base_dst)
+            base_clocks = sampler.stop() if sampler else None
             base = {"impl": "cuBLAS + NCCL all_gather_into_tensor", "ms_per_step": round(base_ms, 4),
-                    "tflops": round(2.0 * M * N * K / (base_ms * 1e-3) / 1e12, 1), "per_step_ms": bst,
+                    "tflops": round(2.0 * M * N * K / (base_ms * 1e-3) / 1e12, 1), "per_step_ms": bst, "clocks": base_clocks,
                     "e2e": {"ms_per_step": round(base_e2e_ms, 4),
                             "value": round(2.0 * M * N * K / (base_e2e_ms * 1e-3) / 1e12, 2), "unit": "TFLOP/s",
                             "h2d_bytes_per_step": h2d_bytes, "d2h_bytes_per_step": rows_host[0].numel() * 2}}
