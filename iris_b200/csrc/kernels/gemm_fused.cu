@@ -1462,109 +1462,122 @@ const char* iris_gemm_last_error() { return g_err; }
 int iris_gemm_smem_bytes() { return kSmemBytes; }
 int iris_gemm_desc_size() { return (int)sizeof(IrisGemmDesc); }
 
-void* iris_gemm_plan_create(const IrisGemmDesc* d) {
+// Whether the sizes, the element type and the schedule of a description are ones the kernels take: 0, or -1 with a message
+// in iris_gemm_last_error().  Looks at no device and no buffer; iris_gemm_plan_create begins with it.
+int iris_gemm_plan_check(const IrisGemmDesc* d) {
   g_err[0] = 0;
   if (d->world < 1 || d->world > kMaxRanks || d->num_local < 1 || d->num_local > kMaxRanks) {
     snprintf(g_err, sizeof(g_err), "world and num_local must be in [1, %d]", kMaxRanks);
-    return nullptr;
+    return -1;
   }
   if (d->M < 1 || d->N < 1 || d->K < 1) {
     snprintf(g_err, sizeof(g_err), "M, N, K must be positive");
-    return nullptr;
+    return -1;
   }
   if (d->dtype < kBf16 || d->dtype > kInt8) {
     snprintf(g_err, sizeof(g_err), "element type must be bf16 (0), fp16 (1), fp32 multiplied as tf32 (2) or int8 (3)");
-    return nullptr;
+    return -1;
   }
   const int et = d->dtype;
   const int es = elem_size(et);
   const int epi_cols = 128 / es;  // columns of an epilogue sub-tile (128-byte rows)
   if ((d->N * es) % 16 != 0 || (d->K * es) % 16 != 0) {
     snprintf(g_err, sizeof(g_err), "rows of N and of K elements must be multiples of 16 bytes");
-    return nullptr;
+    return -1;
   }
   if (d->world > 1 && d->store_all && d->N % epi_cols != 0) {
     snprintf(g_err, sizeof(g_err), "N per rank must be a multiple of %d when tiles are pushed to peers", epi_cols);
-    return nullptr;
+    return -1;
   }
   if (es != 2 && (d->mode != kEpiStore || d->sk_units > 0 || d->ksplit > 1)) {
     snprintf(g_err, sizeof(g_err), "fp32 and int8 matrices: store mode with whole tiles only (plain GEMM, all-scatter, "
                                    "all-gather prologue)");
-    return nullptr;
+    return -1;
   }
   const int cg = d->cta_group == 2 ? 2 : 1;
   const int bn = d->bn > 0 ? d->bn : BN;
   if (bn != 64 && bn != 128 && bn != 256) {
     snprintf(g_err, sizeof(g_err), "tile width must be 64, 128 or 256 columns");
-    return nullptr;
+    return -1;
   }
   if (bn % epi_cols != 0) {
     snprintf(g_err, sizeof(g_err), "tile width must be a multiple of %d columns for this element type", epi_cols);
-    return nullptr;
+    return -1;
   }
   const int tail_split = d->tail_tiles > 0 && d->tail_split > 1 ? d->tail_split : 1;
-  const int tail_tiles = tail_split > 1 ? d->tail_tiles : 0;
   if (tail_split > 1) {
     const bool plain = (d->mode == kEpiStore || d->mode == kEpiReduce) && d->sk_units <= 0 && d->ksplit <= 1;
     if (!plain || bn % tail_split != 0 || (bn / tail_split) % epi_cols != 0 || ((bn / tail_split) / cg) % 8 != 0) {
       snprintf(g_err, sizeof(g_err), "a column-split tail needs store / reduce mode, whole tiles and pieces of whole "
                                      "%d-column sub-tiles", epi_cols);
-      return nullptr;
+      return -1;
     }
   }
   if (d->push_kind < kPushTma || d->push_kind > kPushMultimem) {
     snprintf(g_err, sizeof(g_err), "push_kind must be 0..3");
-    return nullptr;
+    return -1;
   }
   if (d->push_kind == kPushStores && d->mode == kEpiReduce) {
     snprintf(g_err, sizeof(g_err), "push_kind 2 (plain stores) cannot add: use 0, 1 or 3 with mode reduce");
-    return nullptr;
+    return -1;
   }
   if (d->push_kind == kPushMultimem && d->world > 1 && d->store_all &&
       (d->mode == kEpiStore || d->mode == kEpiReduce) && d->mc_base == 0) {
     snprintf(g_err, sizeof(g_err), "push_kind 3 (multimem) needs a heap bound to an NVLS multicast object");
-    return nullptr;
+    return -1;
   }
   if (d->rs_rows > 0) {
     const int gm = d->group_m < 1 ? 1 : d->group_m;
     if (d->mode != kEpiOneShot || !d->push_partials || d->ksplit > 1 || d->sk_units > 0) {
       snprintf(g_err, sizeof(g_err), "reduce-scatter runs as one-shot with pushed partials, whole tiles, no K split");
-      return nullptr;
+      return -1;
     }
     if ((long long)d->rs_rows * d->world != d->M || d->rs_rows % (BM * cg) != 0 || (d->rs_rows / (BM * cg)) % gm != 0) {
       snprintf(g_err, sizeof(g_err), "reduce-scatter needs M = world * rs_rows, rs_rows a multiple of %d x group_m",
                BM * cg);
-      return nullptr;
+      return -1;
     }
     if (d->part_slot_rows < d->rs_rows) {
       snprintf(g_err, sizeof(g_err), "reduce-scatter: inbox slots must hold rs_rows rows");
-      return nullptr;
+      return -1;
     }
     if (d->rs_bcast && d->out_row0 < 0) {
       snprintf(g_err, sizeof(g_err), "push two-shot: the output must be the symmetric one inside the partial matrix");
-      return nullptr;
+      return -1;
     }
   }
   if (d->ag) {
     if (d->M % d->world != 0 || (d->M / d->world) % (BM * cg) != 0) {
       snprintf(g_err, sizeof(g_err), "all-gather prologue needs M / world to be a multiple of %d", BM * cg);
-      return nullptr;
+      return -1;
     }
     if (d->ag_slices < 1 || d->K % d->ag_slices != 0 || (d->K / d->ag_slices * es) % 16 != 0) {
       snprintf(g_err, sizeof(g_err), "ag_slices must divide the rows of K elements into multiples of 16 bytes");
-      return nullptr;
+      return -1;
     }
   }
+  for (int t = 0; t < kMaxRanks; ++t) {
+    if (d->c2_ptr[t] != 0 || d->partial_off[0] != d->partial_off[1]) {
+      snprintf(g_err, sizeof(g_err), "the two partial buffers are row ranges (part_row0) of one matrix per rank");
+      return -1;
+    }
+  }
+  return 0;
+}
+
+void* iris_gemm_plan_create(const IrisGemmDesc* d) {
+  if (iris_gemm_plan_check(d)) return nullptr;
+  const int et = d->dtype;
+  const int es = elem_size(et);
+  const int epi_cols = 128 / es;  // columns of an epilogue sub-tile (128-byte rows)
+  const int cg = d->cta_group == 2 ? 2 : 1;
+  const int bn = d->bn > 0 ? d->bn : BN;
+  const int tail_split = d->tail_tiles > 0 && d->tail_split > 1 ? d->tail_split : 1;
+  const int tail_tiles = tail_split > 1 ? d->tail_tiles : 0;
   cudaSetDevice(d->device);
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->device);
   const bool pull = d->mode == kEpiOneShot || d->mode == kEpiTwoShot;
-  for (int t = 0; t < kMaxRanks; ++t) {
-    if (d->c2_ptr[t] != 0 || d->partial_off[0] != d->partial_off[1]) {
-      snprintf(g_err, sizeof(g_err), "the two partial buffers are row ranges (part_row0) of one matrix per rank");
-      return nullptr;
-    }
-  }
   // Short matrices move short sub-tiles: the C / partial box has only as many rows as M needs (multiple of 8).
   const uint32_t c_box_rows = d->M >= BM ? BM : (uint32_t)((d->M + 7) / 8 * 8);
   int ctas_per_rank = d->ctas_per_rank - d->ctas_per_rank % cg;

@@ -67,6 +67,7 @@ def _lib():
         lib.iris_gemm_last_error.restype = ctypes.c_char_p
         lib.iris_gemm_plan_create.restype = ctypes.c_void_p
         lib.iris_gemm_plan_create.argtypes = [ctypes.POINTER(_Desc)]
+        lib.iris_gemm_plan_check.argtypes = [ctypes.POINTER(_Desc)]
         lib.iris_gemm_plan_destroy.argtypes = [ctypes.c_void_p]
         lib.iris_gemm_plan_ctas_per_rank.argtypes = [ctypes.c_void_p]
         lib.iris_gemm_plan_cta_group.argtypes = [ctypes.c_void_p]
@@ -359,14 +360,14 @@ class FusedGemm:
         d.mc_base = mc if (self.nvls or pk == "multimem") else 0
         self.ag_slices = int(ag_slices)
         lib = _lib()
-        if not self.swiglu:
+        if not self.local:
             self._plan = lib.iris_gemm_plan_create(ctypes.byref(d))
             if not self._plan:
                 raise RuntimeError("fused GEMM plan: " + lib.iris_gemm_last_error().decode())
             self.ctas_per_rank = lib.iris_gemm_plan_ctas_per_rank(self._plan)  # what fits on the device
-        if self.local:   # the fused plan has vetted sizes and schedule (swiglu: checked above); the one-rank kernel runs
-            if not self.swiglu:
-                lib.iris_gemm_plan_destroy(self._plan)
+        else:   # the one-rank kernel; what the fused one refuses stays refused (swiglu: no form of it has that)
+            if not self.swiglu and lib.iris_gemm_plan_check(ctypes.byref(d)) != 0:
+                raise RuntimeError("fused GEMM plan: " + lib.iris_gemm_last_error().decode())
             a0, b0, o0 = a_use[0], bt[0], self.out[0]
             self._plan = lib.iris_gemm_local_create(
                 a0.data_ptr(), a0.stride(0), b0.data_ptr(), b0.stride(0), o0.data_ptr(), o0.stride(0), self.M,

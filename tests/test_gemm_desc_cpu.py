@@ -9,6 +9,7 @@ import pytest
 import torch
 
 import iris_b200 as iris
+from iris_b200 import _native
 from iris_b200.ops import gemm as G
 from iris_b200.ops.gemm_plan import BM, FLAG_HEADER, plan_gemm
 
@@ -277,7 +278,11 @@ class FakeLocalKernels(FakeKernels):
 
     def __init__(self):
         super().__init__()
-        self.local = []
+        self.local, self.checked = [], 0
+
+    def iris_gemm_plan_check(self, ref):
+        self.checked += 1
+        return 0
 
     def iris_gemm_local_create(self, *args):
         self.local.append(dict(zip(("a", "lda", "bt", "ldb", "out", "ldo", "M", "N", "K"), args[:9]), glu=args[-1]))
@@ -316,6 +321,7 @@ def test_one_rank_kernel_only_where_the_output_is_the_product(world1):
     # the adding form clears all of the output, also what lies beside the product
     wide = ctx.zeros((256, 640), dtype=torch.bfloat16)
     assert not G.FusedGemm(ctx, [a], [bt], "reduce", store_all=True, out=[wide]).local
+    fused = len(fake.descs)
     for kw in (dict(mode="store"), dict(mode="store", c_cols=512), dict(mode="reduce", store_all=True),
                dict(mode="reduce", store_all=True, out=[wide[:, :512]]), dict(mode="one_shot"),
                dict(mode="store", out=[wide[:, 64:576]])):
@@ -324,6 +330,7 @@ def test_one_rank_kernel_only_where_the_output_is_the_product(world1):
         got = fake.local[-1]
         assert (got["M"], got["N"], got["K"], got["glu"]) == (256, 512, 128, 0)
         assert got["out"] == op.out[0].data_ptr() and got["ldo"] == op.out[0].stride(0) >= 512
+    assert len(fake.descs) == fused and fake.checked == 6     # no plan of the fused kernel is made only to be thrown away
     op = G.FusedGemm(ctx, [a], [bt], "store", swiglu=True)
     assert op.local and (fake.local[-1]["N"], fake.local[-1]["ldo"], fake.local[-1]["glu"]) == (256, 256, 1)
 
@@ -388,3 +395,31 @@ def test_gemm_checks_its_output_before_the_launch(monkeypatch):
     assert len(calls) == 4
     ctx.backend, ctx.device = "cpu", torch.device("cpu")
     ctx.close()
+
+
+@pytest.mark.skipif(not _native.kernels_available(), reason="native kernels not built")
+def test_plan_check_refuses_without_a_device():
+    """The argument check that a one-rank op makes in place of a plan: the same refusals, and nothing of the device."""
+    lib = G._lib()
+
+    def check(**kw):
+        d = _with(kw)
+        return lib.iris_gemm_plan_check(ctypes.byref(d)), lib.iris_gemm_last_error()
+
+    assert check() == (0, b"")
+    for kw, text in ((dict(M=0), b"positive"), (dict(N=508), b"multiples of 16 bytes"), (dict(K=4), b"multiples of 16 bytes"),
+                     (dict(dtype=7), b"element type"), (dict(dtype=3, mode=G.MODES["reduce"]), b"whole tiles only"),
+                     (dict(bn=96), b"tile width"), (dict(ag=1, M=130), b"all-gather"), (dict(ag=1, K=136, ag_slices=3), b"ag_slices"),
+                     (dict(rs_rows=128, mode=G.MODES["one_shot"]), b"reduce-scatter"), (dict(world=9), b"world"),
+                     (dict(push_kind=9), b"push_kind")):
+        rc, message = check(**kw)
+        assert rc == -1 and text in message, (kw, message)
+        assert not lib.iris_gemm_plan_create(ctypes.byref(_with(kw))) and text in lib.iris_gemm_last_error()
+
+
+def _with(kw):
+    d = G._Desc()
+    for key, value in dict(dict(M=256, N=512, K=128, world=1, num_local=1, mode=G.MODES["store"], bn=256, ag_slices=8,
+                                cta_group=1), **kw).items():
+        setattr(d, key, value)
+    return d
