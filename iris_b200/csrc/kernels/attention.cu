@@ -23,9 +23,9 @@
 //   warp 9          one elected thread issues tcgen05.mma:  S = Q K^T, then O += P V (P from tensor memory, V as an
 //                   MN-major operand: V[key][d] is read as stored), alternating between the sides; the first half of a
 //                   product starts when the first half of P is there
-// What bounds it: the chain of one side, scores -> softmax -> product, about 4500 cycles per step of a pair for 2048 of MMAs
-// and 2048 of ex2 (8 x 2048 tokens x 32 heads from a rest: 317 us causal, 514 without a mask), and in a long run the GPU's
-// power limit (302 - 327 and 575 us back to back).  A scale that is renewed only after a growth of 2^8 takes 287 / 467 us
+// What bounds it: the chain of one side, scores -> softmax -> product: 4300 - 5000 cycles per step of a pair for 2048 of MMAs
+// and 2048 of ex2; in a long run the GPU's power limit takes the clock besides.  8 x 2048 tokens x 32 heads bf16, causal /
+// without a mask: from a rest, 1965 MHz, 317 / 524 us; a run of seconds, 1635 / 1612 MHz at 1010 W, 349 / 585 us.  A scale that is renewed only after a growth of 2^8 takes 287 / 467 us
 // instead, but then a row's largest weight is rounded like the others and the error against 64 bits grows by 2 to 4 %
 // (2.034e-3 -> 2.071e-3, 2.256e-3 -> 2.337e-3, both bf16).
 // Before: one 128-row tile per CTA, two threads per row reading the scores twice, P through shared memory, O folded
@@ -65,8 +65,9 @@ constexpr int kSmemBytes = 1024 + kBarBytes + (2 + kSlots) * kTileBytes;
 static_assert(kSmemBytes <= 227 * 1024, "shared-memory budget");
 
 // The split form, in which the softmax of a tile is part of the chain that sets the time, makes one in so many pairs of
-// exponentials on the FMA units instead of the special-function unit (1 x 4096 x 4 heads causal: 37.3 -> 33.4 us; every
-// third 33.5).  The pair form gains nothing from it (281 -> 285 us).
+// exponentials on the FMA units instead of the special-function unit (1 x 4096 x 4 heads causal: 40.1 -> 38.1 us, 3 x 384 x 5
+// 8.25 -> 8.12, 4 x 3072 x 7 without a mask 172 -> 166 from a rest; 2 x 1024 x 12 loses, 15.1 -> 15.4).  The pair form gains
+// nothing from it.
 constexpr int kPolyEvery = 4;
 
 enum Site : uint32_t { kSiteLoad = 90, kSiteMma = 91, kSiteSoftmax = 92 };
@@ -688,9 +689,9 @@ EncodeTiledFn attn_encode_fn() {
 }
 // Whether the two sides of a CTA share out the keys of one query tile instead of taking two query tiles: if the CTA with
 // the most to do is done clearly earlier.  Time is counted in steps in which both sides do a tile of keys, plus one step
-// per item for its start and its output.  Half the chain is what counts when there are few items: 3 x 384 tokens x 5
-// heads takes 9.3 us with the keys shared out, 2 x 1024 x 12 goes from 23.8 to 15.9 us; with many items the pairs win, because
-// they load every key tile once for 256 queries instead of 128.
+// per item for its start and its output.  Half the chain is what counts when there are few items (pairs -> keys shared out):
+// 3 x 384 tokens x 5 heads 11.7 -> 8.1 us, 2 x 1024 x 12 causal 22.6 -> 15.4, 1 x 4096 x 4 causal 67.2 -> 38.1; with many items
+// the pairs win, because they load every key tile once for 256 queries instead of 128.
 bool split_keys(int batch, int seq, int heads, bool causal, int sms) {
   const long long nq = seq / iris::attn::BQ, bh = (long long)batch * heads;
   auto makespan = [&](bool split) {

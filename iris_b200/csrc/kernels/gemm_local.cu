@@ -18,10 +18,10 @@
 //     (16384 tokens x 11008 x 4096: one pass of 1.08 GB less per layer, the four-layer decoder 22.6 -> 21.7 ms);
 //   * with more tiles than SMs (split 1) a CTA walks over its tiles, two accumulators deep, as the fused kernel does.
 //
-// What bounds it: a few rows, the weights' bytes (1 x 4096 x 11008 bf16: 26.3 us in the fused kernel, 18.4 us here, 4.9 TB/s);
+// What bounds it: a few rows, the weights' bytes (1 x 4096 x 11008 bf16: 26.0 us in the fused kernel, 18.0 us here, 5.0 TB/s);
 // hundreds of rows, loads out of L2 and the number of CTAs (256 x 4096 x 11008: 71 -> 24 us); thousands, the tensor cores
-// and the GPU's power limit (8192 x 14336 x 4096 back to back: 761 -> 703 us, 1.37 PFLOP/s; int8 8192 x 3584 x 14336: 347 ->
-// 297 us; fp32 2048 x 4096 x 4096: 129 -> 110 us).
+// and the GPU's power limit (8192 x 14336 x 4096 back to back: 769 -> 711 us, 1.35 PFLOP/s; int8 8192 x 3584 x 14336: 347 ->
+// 302 us; fp32 2048 x 4096 x 4096: 130 -> 111 us).
 //
 // Roles (320 threads, one CTA per SM): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 epilogue.  The producer starts
 // before the block's set-up barrier (it needs only the ring barriers, which it initialises itself).

@@ -207,10 +207,11 @@ struct MpArgs {
 // chunks still uses the whole GPU.  Block b of a role handles the (chunk, slice) pairs b, b + blocks, ... in order:
 // with blocks = nchunks * parts all chunks travel at once and land together at the end; with fewer blocks the chunks
 // complete one group after the other, and the consumer works on the early ones while the later ones are on the link.
-// Producer: copy the slice into the consumer's buffer, make it visible (barrier + one system-scope fence), count it on
-// the chunk's arrival counter; the block that completes the count raises the CONSUMER's flag with release semantics
-// and puts the counter back to zero.  Consumer: every block of the chunk waits (bounded, acquire) on the chunk's flag
-// in its own memory, then writes out = 2 * landed for its slice.
+// Producer: copy the slice into the consumer's buffer, make it visible (barrier, then one fence of the publishing thread:
+// system scope between GPUs, GPU scope where one launch has both roles), count it with a relaxed add on the chunk's
+// arrival counter; the block that completes the count puts the counter back to zero, fences once more and raises the
+// CONSUMER's flag with a relaxed store, which the fence makes a release.  Consumer: every block of the chunk waits
+// (bounded, acquire) on the chunk's flag in its own memory, then writes out = 2 * landed for its slice.
 //
 // Bound by the chain launch -> copy -> fence -> count -> flag -> copy, not by the 32 MB that 8 chunks of 1 MB move: so all
 // slices are in flight at once (32 registers: 2048 threads per SM, which is both roles' 296 blocks of 512 for that
@@ -270,8 +271,8 @@ __global__ void __launch_bounds__(1024, 2) mp_kernel(MpArgs a) {
         for (size_t i = threadIdx.x; i < bytes / 4; i += blockDim.x)
           store(d + i, load(s + i, a.producer, a.producer, a.hb), a.producer, a.consumer, a.hb);
       }
-      // One thread publishes for the block: the barrier orders every thread's stores before its system-scope fence
-      // (fences are cumulative), and only its warp waits for the link round trip; the others start the next slice.
+      // One thread publishes for the block: the barrier orders every thread's stores before its fence (fences are
+      // cumulative), and only its warp waits for the link round trip; the others start the next slice.
       __syncthreads();
       if (threadIdx.x == 0) {
         fence();

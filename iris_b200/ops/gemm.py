@@ -132,7 +132,7 @@ class FusedGemm:
             ``"two_shot"``.
         store_all: push each tile to every rank (``store`` / ``reduce``).
         c_cols / col_off_per_rank: width of the output buffer and column offset per rank (all-scatter:
-            ``c_cols = world * N``, ``col_off_per_rank = N``).
+            ``c_cols = world * N``, ``col_off_per_rank = N``).  Columns of the product from ``c_cols`` on are not stored.
         ag: run the all-gather prologue (A rows sharded M / world per rank; see ``a_full``).
         reduce_scatter: with ``mode="one_shot"``: every rank keeps only its own ``M / world`` rows of the sum
             (``out[l]`` is that block); partial tiles are pushed to the keeper of their rows only.
@@ -142,10 +142,13 @@ class FusedGemm:
             With ``mode="reduce"`` (atomic all-reduce) ``ksplit`` cuts K into pieces computed by different CTAs that
             all add into the outputs, which spreads a short matrix over the whole GPU.
         nvls: two-shot on a heap bound to an NVLS multicast object: ``None`` = use it when available.
-        trace: record per-tile device timestamps (``trace_records()``).
-        bn: tile width in columns, 64 / 128 / 256 (default 256).  Together with ``cta_group`` (128 or 256 rows) this
-            gives the six tile shapes of the kernel (the reference's per-shape ``BLK_M`` / ``BLK_N``,
-            ``dataset/tiling.json``).
+        trace: record per-tile device timestamps (``trace_records()``).  They are the fused kernel's: with one rank, an op
+            with ``trace=True`` runs that kernel, and one without it the one-rank kernel, which has no trace.
+        bn: tile width of the fused kernel in columns, 64 / 128 / 256 (``None``: 256 there; one rank without an explicit
+            schedule runs a kernel with tile widths of its own).  Together with ``cta_group`` (128 or 256 rows) this gives
+            the six tile shapes of the kernel (the reference's per-shape ``BLK_M`` / ``BLK_N``, ``dataset/tiling.json``).
+        stream_k: the fused kernel's stream-K schedule.  With this argument or with ``IRIS_STREAM_K`` in the environment,
+            one rank runs the fused kernel too.
         tail_split: cut the tiles of a ragged last wave into column pieces: ``True`` = two, an integer = at most that
             many (store / reduce modes, whole-tile schedule; default off).
         push_kind: how tiles travel in the all-scatter and atomic all-reduce forms: ``"tma"`` (one thread issues a TMA
@@ -571,8 +574,10 @@ def _stream_object(device: int, raw: int) -> "torch.cuda.Stream":
 def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
          cta_group: Optional[int] = None, bn: Optional[int] = None, tail_split: Optional[bool] = None) -> torch.Tensor:
     """Single-GPU ``a @ bt.T`` on the tcgen05 kernel (world of one, no communication): bf16, fp16, float32 (as tf32)
-    or int8 (the low 8 bits of the integer sums).  Runs in stream order on the current stream; with an explicit schedule
-    (``cta_group``, ``bn``, ``tail_split``) it builds and releases a :class:`FusedGemm` and waits for it."""
+    or int8 (the low 8 bits of the integer sums).  Runs in stream order on the current stream, like any PyTorch operator: the
+    host does not wait, and another stream that reads the result has to wait for this one (an event, ``wait_stream``).
+    With an explicit schedule (``cta_group``, ``bn``, ``tail_split``) it builds and releases a :class:`FusedGemm` and waits
+    for it.  ``out`` may be larger than the product, which takes its first rows and columns."""
     dev = a.device
     ctx = _private_ctx.get(dev)
     if ctx is None:
