@@ -665,7 +665,7 @@ int resident_groups(int c, int sms) {
 // the smallest estimated time.  The estimate (in us; without what every combination has) has one term for each thing that
 // was found to bind somewhere; its constants are a fit to 14600 timings of 330 products (1 .. 16384 rows, all four types) in
 // CUDA graphs.  Over those the chosen combination takes 2.6 % more than the fastest one on average, 37 % at worst (a 5 us
-// product).
+// product); over 110 products drawn afterwards 3.6 % (median 0.4 %, one in ten more than 13 %), 34 % at worst (K of two blocks).
 //   * a K block (128 bytes of K) takes the longest of: the MMAs, 2 cycles per column of the tile; 340 - 400 cycles of issue;
 //     the 1.4 us from one use of a ring slot to the next, shared by the ring's stages; the loads of all SMs at 19 TB/s out
 //     of L2.  Rows that do not start on 128 bytes touch one more L2 line each (12 % and 22 % on the last two), and rows past
