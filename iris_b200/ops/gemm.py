@@ -121,6 +121,13 @@ def as_kmajor_bt(b: torch.Tensor) -> torch.Tensor:
     raise ValueError("B must be K-contiguous (pass randn(n, k).T or an [N, K] tensor)")
 
 
+def _asks_for_fused(options: dict) -> bool:
+    """Whether the options of an op name a schedule of the fused kernel, or its trace."""
+    return (bool(options.get("trace")) or bool(options.get("nvls")) or "IRIS_STREAM_K" in os.environ or any(
+        options.get(name) is not None for name in ("ctas_per_rank", "group_m", "cta_group", "stream_k", "push", "ksplit", "bn",
+                                                   "tail_split", "push_kind")))
+
+
 class FusedGemm:
     """One fused GEMM + collective on fixed buffers.
 
@@ -226,8 +233,7 @@ class FusedGemm:
         whole = self.swiglu or mode in ("one_shot", "two_shot") or not c_cols or int(c_cols) == self.N
         if mode == "reduce" and out is not None and tuple(out[0].shape) != (self.M, self.N):
             whole = False
-        self.local = (self.world == 1 and whole and not trace and not nvls and "IRIS_STREAM_K" not in os.environ and all(
-            x is None for x in (ctas_per_rank, group_m, cta_group, stream_k, push, ksplit, bn, tail_split, push_kind)))
+        self.local = self.world == 1 and whole and not _asks_for_fused(self._ctor[4])
         if self.local:
             stream_k = False
         if self.swiglu:
@@ -530,8 +536,11 @@ def gemm_all_reduce(ctxs, a, bt, variant: str = "one_shot", **kw) -> FusedGemm:
     to every rank; needs ``M`` to be a multiple of ``world x 128``)."""
     if variant == "auto":
         variant, auto_kw = auto_all_reduce_variant(a[0].shape[0], world_of(ctxs))
-        # (one rank has nothing to reduce: the op picks its own schedule, see FusedGemm)
-        kw = dict(auto_kw, **kw) if world_of(ctxs) > 1 else kw
+        # (one rank has nothing to reduce: the op runs the one-rank kernel, unless these options rule that out, see FusedGemm)
+        out, n = kw.get("out"), as_kmajor_bt(bt[0]).shape[0]
+        if world_of(ctxs) > 1 or _asks_for_fused(kw) or int(kw.get("c_cols") or n) != n or (
+                variant == "atomic" and out is not None and tuple(out[0].shape) != (a[0].shape[0], n)):
+            kw = dict(auto_kw, **kw)
     if variant == "atomic":
         return FusedGemm(ctxs, a, bt, "reduce", store_all=True, **kw)
     if variant in ("one_shot", "two_shot"):

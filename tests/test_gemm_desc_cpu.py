@@ -3,6 +3,7 @@ library that records the descriptor and the launch arguments.  Checks the packin
 collective, the buffer layout on the heap, and the cumulative per-call targets; and the pure planner
 (``iris_b200/ops/gemm_plan.py``) over many shapes."""
 import ctypes
+import gc
 from types import SimpleNamespace
 
 import pytest
@@ -304,6 +305,8 @@ def world1(monkeypatch):
     monkeypatch.delenv("IRIS_STREAM_K", raising=False)
     ctx.backend = "cuda"
     yield ctx, fake
+    for op in [o for o in gc.get_objects() if isinstance(o, G.FusedGemm)]:
+        op._plan = None    # a test that failed keeps its ops: their stand-in handles must not reach the library
     ctx.backend = "cpu"
     ctx.close()
 
@@ -333,6 +336,21 @@ def test_one_rank_kernel_only_where_the_output_is_the_product(world1):
     assert len(fake.descs) == fused and fake.checked == 6     # no plan of the fused kernel is made only to be thrown away
     op = G.FusedGemm(ctx, [a], [bt], "store", swiglu=True)
     assert op.local and (fake.local[-1]["N"], fake.local[-1]["ldo"], fake.local[-1]["glu"]) == (256, 256, 1)
+
+
+def test_automatic_all_reduce_keeps_its_schedule_beside_options(world1):
+    """With one rank and an option that asks for the fused kernel, ``variant="auto"`` still cuts K of a short matrix into
+    pieces; without one the op runs the one-rank kernel."""
+    ctx, fake = world1
+    (a,), (bt,) = _ab(1, 512, 2048, 1)
+    plain = G.gemm_all_reduce(ctx, [a], [bt], variant="auto", timeout_ms=500.0)
+    assert plain.local and plain.mode == "reduce"
+    wide = ctx.zeros((1, 640), dtype=torch.bfloat16)
+    for kw in (dict(cta_group=1), dict(group_m=4), dict(trace=True), dict(c_cols=256), dict(out=[wide])):
+        op = G.gemm_all_reduce(ctx, [a], [bt], variant="auto", **kw)
+        assert not op.local and op.ksplit == 8 and fake.descs[-1].ksplit == 8, kw
+    assert G.gemm_all_reduce(ctx, [a], [bt], variant="auto", ksplit=2).ksplit == 2
+    assert G.gemm_all_reduce(ctx, [a], [bt], variant="auto", out=[wide[:, :512]]).local
 
 
 def test_outputs_and_devices_are_checked_before_any_launch(world1, monkeypatch):
