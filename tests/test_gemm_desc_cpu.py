@@ -305,7 +305,7 @@ def world1(monkeypatch):
     monkeypatch.delenv("IRIS_STREAM_K", raising=False)
     ctx.backend = "cuda"
     yield ctx, fake
-    for op in [o for o in gc.get_objects() if isinstance(o, G.FusedGemm)]:
+    for op in [o for o in gc.get_objects() if type(o) is G.FusedGemm]:
         op._plan = None    # a test that failed keeps its ops: their stand-in handles must not reach the library
     ctx.backend = "cpu"
     ctx.close()
