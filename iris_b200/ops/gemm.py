@@ -596,17 +596,18 @@ def gemm(a: torch.Tensor, bt: torch.Tensor, out: Optional[torch.Tensor] = None,
     bt = as_kmajor_bt(bt)
     n = bt.shape[0]
     device = a.get_device()
-    if out is None:
+    given = out is not None
+    if not given:
         out = a.new_empty((a.shape[0], n))
     if (cta_group is None and bn is None and tail_split is None and "IRIS_STREAM_K" not in os.environ
-            and bt.get_device() == device and out.get_device() == device):
+            and bt.get_device() == device and (not given or out.get_device() == device)):
         _check_operand(bt, "B")
         _check_operand(a, "A", bt.dtype)
         m, k = a.shape
         if k != bt.shape[1]:
             raise ValueError(f"K mismatch: A has {k}, B has {bt.shape[1]}")
         _check_operand(out, "output", bt.dtype)
-        if out.shape[0] < m or out.shape[1] < n:
+        if given and (out.shape[0] < m or out.shape[1] < n):
             raise ValueError(f"output: [{m}, {n}] or larger, got {tuple(out.shape)}")
         raw = _native.current_stream(device)
         lib = _lib()
